@@ -339,9 +339,10 @@ def work(case):
 
 
 def tolerance(case):
-    """bf16 activations throughout; the fp8 model rounds them to e4m3 in front of every product as well, so that a last bit of
-    bf16 turns into a step of e4m3 here and there."""
-    return {"rel": 0.03 if case["family"] == "latent" else 0.02, "max": 0.3}
+    """bf16 activations throughout: against 64 bits a step is off by 0.005 (experts: the routers' margins carry the embedding
+    through), 0.011 (dense), 0.017 (hybrid) and 0.05 (latent, whose fp8 products also round activations to e4m3), and another
+    correct order of sums or roundings by about as much from this one, except that roundings of the same inputs are shared."""
+    return {"rel": 0.02 if case["family"] == "moe" else 0.03, "max": 0.3}
 
 
 # ----------------------------------------------------------------------------- the same in 64 bits
