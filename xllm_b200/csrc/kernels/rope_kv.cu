@@ -13,7 +13,7 @@
 namespace xllm {
 
 struct RopeKvParams {
-  const bf16* qkv;      // [T, (nq + 2*nkv) * d]
+  const bf16* qkv;      // [T, nq * q_hs + 2*nkv*d]
   int64_t qkv_stride;   // elements between token rows
   bf16* q_out;          // [T, nq, d]
   bf16* k_cache;        // paged, may be null
@@ -26,7 +26,8 @@ struct RopeKvParams {
   const int64_t* positions;  // [T]
   const int32_t* slots;      // [T] (block*block_size + offset; <0 skips the cache write), may be null
   int tokens, nq, nkv, d, rot, block_size, interleaved;
-  float eps;
+  int q_hs;                  // elements between query heads (2 d where each lies beside its output gate)
+  float eps, w_offset;       // the norm weights are w + w_offset
 };
 
 // One CTA per token.  A thread owns the same 8-element slot of up to kRopeHeadsPerThread heads (the
@@ -74,7 +75,7 @@ __global__ void __launch_bounds__(256) rope_kv_kernel(RopeKvParams p) {
 #pragma unroll
     for (int u = 0; u < kRopeHeadsPerThread; ++u) {
       const int h = h0 + u * heads_per_pass + local;
-      if (h < total_heads) raw[u] = reinterpret_cast<const bf16x8*>(row + (int64_t)h * p.d)[g];
+      if (h < total_heads) raw[u] = reinterpret_cast<const bf16x8*>(row + (int64_t)min(h, p.nq) * p.q_hs + max(h - p.nq, 0) * p.d)[g];
     }
 #pragma unroll
     for (int u = 0; u < kRopeHeadsPerThread; ++u) {
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(256) rope_kv_kernel(RopeKvParams p) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             // match the usual bf16 module: normalise, round to bf16, scale by the bf16 weight
-            x[j] = __bfloat162float(__float2bfloat16(x[j] * inv)) * w[j];
+            x[j] = __bfloat162float(__float2bfloat16(x[j] * inv)) * (w[j] + p.w_offset);
           }
         }
       }
@@ -157,11 +158,11 @@ XLLM_API int xllm_rope_kv(const void* qkv, int64_t qkv_stride, void* q_out, void
                           void* v_cache, void* k_out, void* v_out, const void* q_norm_w,
                           const void* k_norm_w, const void* cos_sin, const void* positions,
                           const void* slots, int tokens, int nq, int nkv, int d, int rot,
-                          int block_size, int interleaved, float eps, void* stream) {
+                          int block_size, int interleaved, float eps, int q_hs, float w_offset, void* stream) {
   using namespace xllm;
   if (tokens == 0) return 0;
   const int tph = d >> 3;
-  if (d % 8 != 0 || tph > 32 || (tph & (tph - 1)) != 0) return (int)cudaErrorInvalidValue;
+  if (q_hs < d || q_hs % 8 != 0 || d % 8 != 0 || tph > 32 || (tph & (tph - 1)) != 0) return (int)cudaErrorInvalidValue;
   if (cos_sin && !interleaved) {
     const int hl = (rot >> 1) >> 3;
     if (hl == 0 || (hl & (hl - 1)) != 0 || rot > d) return (int)cudaErrorInvalidValue;
@@ -172,7 +173,7 @@ XLLM_API int xllm_rope_kv(const void* qkv, int64_t qkv_stride, void* q_out, void
   p.q_norm_w = (const bf16*)q_norm_w; p.k_norm_w = (const bf16*)k_norm_w;
   p.cos_sin = (const float*)cos_sin; p.positions = (const int64_t*)positions;
   p.slots = (const int32_t*)slots; p.tokens = tokens; p.nq = nq; p.nkv = nkv; p.d = d; p.rot = rot;
-  p.block_size = block_size; p.interleaved = interleaved; p.eps = eps;
+  p.block_size = block_size; p.interleaved = interleaved; p.eps = eps; p.q_hs = q_hs; p.w_offset = w_offset;
   // float4 loads of the cos / sin rows: `rot` floats per position, 8-element slots
   if (cos_sin && (rot % 8 != 0 || ((uintptr_t)cos_sin & 15))) return (int)cudaErrorInvalidValue;
   launch_pdl(rope_kv_kernel, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, p);

@@ -510,7 +510,9 @@ class Attention(Module):
     def forward(self, x, positions, meta: AttentionMetadata, k_cache, v_cache):
         return self._attend(self.qkv(x), positions, meta, k_cache, v_cache)
 
-    def _attend(self, qkv, positions, meta: AttentionMetadata, k_cache, v_cache, gate=None):
+    def _attend(self, qkv, positions, meta: AttentionMetadata, k_cache, v_cache, gate=None, q_head_stride=None):
+        """`gate`: the output's gate [T, heads * d], or, with `q_head_stride`, a view of the rows of `qkv` that starts at head
+        0's gate and has the heads that far apart, as their queries are."""
         cos_sin = self.rope.cos_sin
         if meta.rope_table is not None:
             cos_sin, positions = meta.rope_table, meta.rope_rows
@@ -530,8 +532,9 @@ class Attention(Module):
             return self.o_proj(out)
         q = ops.rope_kv_write(qkv, self.nq, self.nkv, self.d, positions, cos_sin, self.rope.rot_dim,
                               slots=meta.slots, k_cache=k_cache, v_cache=v_cache,
-                              q_norm_w=self._norm_w(self.q_norm), k_norm_w=self._norm_w(self.k_norm), eps=self.eps,
-                              interleaved=self.rope.interleaved)
+                              q_norm_w=getattr(self.q_norm, "weight", None), k_norm_w=getattr(self.k_norm, "weight", None),
+                              eps=self.eps, interleaved=self.rope.interleaved, q_head_stride=q_head_stride,
+                              norm_offset=1.0 if self.q_norm is not None and self.q_norm.gemma else 0.0)
         if meta.kv_hook is not None:
             meta.kv_hook(k_cache)
         T = q.shape[0]
@@ -546,8 +549,12 @@ class Attention(Module):
             ops.paged_prefill_attention(q, k_cache, v_cache, meta.block_table[nd:], meta.cu_q[nd:],
                                         meta.kv_lens[nd:], meta.max_q_len, self.scale, causal=True,
                                         window=self.window, out=out)
+        if q_head_stride is not None:                      # per-element output gate (Qwen3-Next)
+            from ..ops import gdn
+            gdn.sigmoid_gate_(out, gate, q_head_stride)
+            gate = None
         out = out.view(T, self.nq * self.d)
-        if gate is not None:                               # per-element output gate (Qwen3-Next)
+        if gate is not None:
             out = out * torch.sigmoid(gate.float()).to(out.dtype)
         return self.o_proj(out)
 

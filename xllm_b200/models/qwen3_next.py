@@ -12,8 +12,8 @@ the state updates they cause.
 
 Parity: xllm/models/llm/qwen3_next.h and the `LinearState` block manager of the reference
 (xllm/core/framework/block/); the arithmetic follows the published HuggingFace implementation, which
-is the oracle of the CPU test.  The recurrence runs on tensor-library ops (one batched update per
-decode step, a token loop per prompt chunk); a fused kernel for it is not built.
+is the oracle of the CPU test.  On CUDA in bf16 a layer's work between its projections is ops/gdn.GatedDelta, driven by
+device inputs alone, so that whole steps are captured; other types and sizes run on tensor-library operations.
 """
 from __future__ import annotations
 
@@ -72,14 +72,28 @@ class GatedDeltaNet(Module):
         self.norm_w = self.add_param("norm.weight", torch.ones(self.dv, dtype=dtype, device=device))
         self.out_proj = self.add_module("out_proj", Linear(self.value_dim, H, False, dtype, device))
 
-    def _step(self, S, q, k, v, g, beta):
-        """One token for a batch of states: S [B, nv, dk, dv]; q, k [B, nv, dk]; v [B, nv, dv]; g, beta [B, nv]."""
-        S = S * g.exp()[:, :, None, None]
-        delta = (v - (S * k[..., None]).sum(-2)) * beta[..., None]
-        S = S + k[..., None] * delta[:, :, None, :]
-        return S, (S * q[..., None]).sum(-2)
+        self.fused = None
+        if gdn_ops.layer_supported(dtype, device, self.nk, self.nv, self.dk, self.dv, self.K):
+            self.fused = gdn_ops.GatedDelta(self.nk, self.nv, self.dk, self.dv, self.K, self.eps, self.conv_w, self.dt_bias,
+                                            self.A_log, self.norm_w)
+
+    def _forward_fused(self, x, meta, state: LinearStateCache):
+        nk, nv, dk, dv, r = self.nk, self.nv, self.dk, self.dv, self.nv // self.nk
+        if self.split_proj:
+            y, z, b, a = self.in_proj_qkv(x), self.in_proj_z(x), self.in_proj_b(x), self.in_proj_a(x)
+            k, v, strides = y[:, self.key_dim:], y[:, 2 * self.key_dim:], (dk, r * dv, r * dv, r)
+        else:
+            y, b = self.in_proj_qkvz(x), self.in_proj_ba(x)
+            k, v, z, a = y[:, dk:], y[:, 2 * dk:], y[:, 2 * dk + r * dv:], b[:, r:]
+            width = 2 * dk + 2 * r * dv
+            strides = (width, width, width, 2 * r)
+        out = self.fused(state.rec[self.lin_idx], state.conv[self.lin_idx], meta.state_slots, meta.cu_q, meta.kv_lens,
+                         meta.n_decode, y, k, v, z, b, a, *strides)
+        return self.out_proj(out)
 
     def forward(self, x, meta, state: LinearStateCache):
+        if self.fused is not None:
+            return self._forward_fused(x, meta, state)
         T = x.shape[0]
         nk, nv, dk, dv, r = self.nk, self.nv, self.dk, self.dv, self.nv // self.nk
         if self.split_proj:
@@ -96,7 +110,9 @@ class GatedDeltaNet(Module):
         beta = torch.sigmoid(b.reshape(T, nv).float())
         g = -self.A_log.float().exp() * F.softplus(a.reshape(T, nv).float() + self.dt_bias.float())
         conv, rec = state.conv[self.lin_idx], state.rec[self.lin_idx]
-        slots, fresh, bounds = meta.state_slots, meta.state_fresh, meta.seq_bounds
+        cu, lens, slots = meta.cu_q.tolist(), meta.kv_lens.tolist(), meta.state_slots.long()
+        bounds = list(zip(cu[:-1], cu[1:]))
+        fresh = [n == e - b for (b, e), n in zip(bounds, lens)]
         out = torch.empty(T, nv, dv, dtype=torch.float32, device=x.device)
 
         def heads(y):                                      # conv output rows -> normalised, scaled q / k and v per value head
@@ -112,6 +128,9 @@ class GatedDeltaNet(Module):
         nd = meta.n_decode
         if nd > 0:                                         # one token per sequence: a single batched update
             s = slots[:nd]
+            for i in range(nd):                            # a prompt of one token starts from zeros
+                if fresh[i]:
+                    conv[s[i]], rec[s[i]] = 0, 0
             tail = conv[s]                                 # [B, conv_dim, K-1]
             full = torch.cat([tail, mixed[:nd, :, None]], dim=-1)                     # [B, conv_dim, K]
             y = F.silu((full.float() * self.conv_w.float()).sum(-1)).to(x.dtype)
@@ -153,6 +172,8 @@ class GatedAttention(Attention):
     def forward(self, x, positions, meta, k_cache, v_cache):
         T, nq, d = x.shape[0], self.nq, self.d
         qkv = self.qkv(x)
+        if qkv.is_cuda and meta.xattn is None:             # queries and gates are read where the projection left them
+            return self._attend(qkv, positions, meta, k_cache, v_cache, gate=qkv[:, d:], q_head_stride=2 * d)
         qg = qkv[:, : nq * d * 2].view(T, nq, 2 * d)
         gate = qg[..., d:].reshape(T, nq * d)
         packed = torch.cat([qg[..., :d].reshape(T, nq * d), qkv[:, nq * d * 2:]], dim=-1)
@@ -193,7 +214,7 @@ class NextDecoderLayer(DecoderLayer):
 class Qwen3NextCausalLM(DenseCausalLM):
     fused_tp = False
     needs_state = True
-    supports_graph = False
+    state_on_device = True          # state slots are a device input of the step: graphs capture it
 
     def __init__(self, args, dtype=torch.bfloat16, device="cpu", ps=None):
         e = dict(args.extra)
@@ -217,6 +238,10 @@ class Qwen3NextCausalLM(DenseCausalLM):
             if not layer.linear:
                 layer.mixer.q_norm.gemma = layer.mixer.k_norm.gemma = True
         self.state = None
+
+    @property
+    def supports_graph(self):
+        return all(l.mixer.fused is not None for l in self.layers if l.linear)
 
     @property
     def num_kv_heads_local(self):

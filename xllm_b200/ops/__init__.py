@@ -108,16 +108,22 @@ def silu_and_mul(x, out=None):
 # ----------------------------------------------------------------------------- rope + kv write
 def rope_kv_write(qkv, nq, nkv, d, positions, cos_sin, rot, slots=None, k_cache=None, v_cache=None,
                   q_norm_w=None, k_norm_w=None, eps=1e-6, interleaved=False, q_out=None,
-                  return_kv=False):
-    """Per-head RMSNorm (optional) + RoPE on packed QKV, K/V scattered into the paged cache.
+                  return_kv=False, q_head_stride=None, norm_offset=0.0):
+    """Per-head RMSNorm (optional) + RoPE on packed QKV, K/V scattered into the paged cache.  `q_head_stride`: elements
+    between query heads where something lies behind each (default d: nothing); the norm weights are w + `norm_offset`.
 
     Returns q [T, nq, d] (and dense k, v when return_kv)."""
     T = qkv.shape[0]
+    qs = q_head_stride or d
     if _debug.enabled():
         _debug.check_range(positions, 0, cos_sin.shape[0], "rope_kv_write positions")
         if k_cache is not None and slots is not None:
             _debug.check_range(slots, 0, k_cache.shape[0] * k_cache.shape[2], "rope_kv_write slots", allow_negative_skip=True)
     if not qkv.is_cuda:
+        if qs != d:
+            qkv = torch.cat([qkv[:, :nq * qs].reshape(T, nq, qs)[..., :d].reshape(T, nq * d), qkv[:, nq * qs:]], dim=-1)
+        if norm_offset:
+            q_norm_w, k_norm_w = (None if w is None else w + norm_offset for w in (q_norm_w, k_norm_w))
         q, k, v = reference.rope_kv(qkv, nq, nkv, d, positions, cos_sin, rot, q_norm_w, k_norm_w,
                                     eps, interleaved)
         if k_cache is not None and slots is not None:
@@ -137,7 +143,7 @@ def rope_kv_write(qkv, nq, nkv, d, positions, cos_sin, rot, slots=None, k_cache=
     check(_lib_().xllm_rope_kv(ptr(qkv), qkv.stride(0), ptr(q_out), ptr(k_cache), ptr(v_cache),
                                ptr(k_out), ptr(v_out), ptr(q_norm_w), ptr(k_norm_w), ptr(cos_sin),
                                ptr(positions), ptr(slots), T, nq, nkv, d, rot, page,
-                               int(interleaved), eps, stream()), "rope_kv")
+                               int(interleaved), eps, qs, norm_offset, stream()), "rope_kv")
     _count()
     return (q_out, k_out, v_out) if return_kv else q_out
 

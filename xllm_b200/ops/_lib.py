@@ -99,7 +99,7 @@ def _declare(lib):
         "xllm_rmsnorm": [P, P, P, P, I, I, F, L, L, I, P],
         "xllm_rmsnorm_static_fp8": [P, P, P, P, P, I, I, F, P],
         "xllm_act_and_mul": [P, P, L, I, L, I, F, F, P],
-        "xllm_rope_kv": [P, L, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, P],
+        "xllm_rope_kv": [P, L, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, F, P],
         "xllm_paged_decode_attn": [P, P, L, P, P, P, I, P, I, I, I, I, I, F, I, P, P],
         "xllm_paged_decode_attn_window": [P, P, L, P, P, P, I, P, I, I, I, I, I, F, I, P, I, P],
         "xllm_paged_decode_attn_kept": [P, P, L, P, P, P, I, P, I, I, I, I, I, F, I, P, I, I, F, P],
