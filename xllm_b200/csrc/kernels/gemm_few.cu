@@ -1,0 +1,442 @@
+// Products of few rows (decode: up to 64), C[M, N] (bf16) = A[M, K] W[N, K]^T, whose time is the weights' way from HBM:
+//
+//   bf16               (+ bias), the contract of xllm_gemm_bf16
+//   block-scaled fp8   sum over 128-wide K blocks of (A_q . W_q^T) a_scale[m, kb] w_scale[n / 128, kb], A_q, W_q e4m3, sums in
+//                      fp32: that of xllm_gemm_fp8_block
+//   grouped (experts)  either, rows of A sorted by expert in tiles of TN rows, tile_expert as in gemm_tcgen05.cu; bf16 also
+//                      with the gated activation of interleaved gate and up rows
+//
+// The operands are swapped: 128 WEIGHT rows are the rows of the tcgen05 tile and 16, 32 or 64 token rows its columns, so what
+// is read back (per K block for fp8, whose blocks differ in scale) is the tokens there are, not 128 columns of weights for a
+// tile of mostly absent rows, and an expert with four rows costs no loads and stores of 128.  A CTA needs half an SM, and two
+// of them cover each other's start and end.  Where the tiles alone leave SMs idle, a cluster of up to eight CTAs cuts K:
+// every CTA sums its slice, the slices meet through distributed shared memory, in a fixed order.  (Split-K in
+// gemm_tcgen05.cu meets in scratch memory by reduce-adds, a round trip of some 6 us.)  The first weights of an ungrouped
+// product start for L2 before the wait for the kernel in front.
+//
+// Measured (one B200, 16 rows, before: gemm_fp8_block_kernel): 7168 x 16384 fp8 (117 MB of weights, 18 us at the copy rate)
+// 55 -> 27 us, 1536 x 7168 24 -> 7 us, 7168 x 18432 58 -> 26 us; 32 experts' 4096 x 7168 and 7168 x 2048 fp8 190 -> 126 us and
+// 210 -> 63 us.  bf16, one row (before: split-K in gemm_tcgen05.cu, and the activation's own kernel): 4096 x 4096 13 -> 9 us,
+// gated 24576 x 4096 44 -> 39 us (31 at the copy rate), 4096 x 12288 26 -> 20 us.
+//
+// Every mbarrier wait is bounded; on expiry all roles leave, tensor memory is released and an error word is set
+// (xllm_gemm_few_error_status).
+#include "tc_common.cuh"
+#include <atomic>
+
+namespace xllm {
+namespace few {
+
+using namespace tc;
+
+constexpr int kAcc = 4, kMaxSplit = 8, kPrefetchBlocks = 8;
+
+template <int TN, bool FP8>
+struct Smem {
+  static constexpr int cols = FP8 ? kAcc * TN : (TN < 32 ? 32 : TN);   // of tensor memory
+  static constexpr int stages = TN == 64 ? 3 : 4;
+  static constexpr int w_bytes = 128 * 128, x_bytes = TN * 128, stage = w_bytes + x_bytes;
+  static constexpr int bars = stages * stage, scales = bars + (2 * stages + 2 * kAcc) * 8 + 16;
+  static constexpr int total(int k_blocks) { return scales + (FP8 ? k_blocks * TN * 4 : 0) + 1024; }
+  static_assert(stage % 1024 == 0 && 2 * TN * 128 * 4 <= stages * stage, "the sums meet where the ring was");
+};
+
+struct Params {
+  bf16* c;
+  int64_t ldc;
+  const float *a_scale, *w_scale;      // fp8
+  const bf16* bias;                    // bf16, or null
+  int M, N, k_blocks, x_rows;          // k_blocks of 128 bytes; x_rows: rows of a copy of A
+  const int32_t* tile_expert;
+  int act;                             // 0, or as in GemmMode: W's rows are [64 gate | 64 up], C has N / 2 columns
+  float limit, alpha;
+  int* err;
+};
+
+// kind::f8f6f4, A = B = e4m3 (both K-major), D = f32, M = 128
+__device__ __forceinline__ void umma_fp8(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(id), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void prefetch_2d(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {
+  float v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}"
+               : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ float gated(float x, float y, int act, float limit, float alpha) {
+  if (act == 4) return clamped_glu(x, y, limit, alpha);
+  if (act == 1) return x / (1.f + __expf(-x)) * y;
+  if (act == 2) return 0.5f * x * (1.f + erff(x * 0.70710678f)) * y;
+  return 0.5f * x * (1.f + tanhf(0.7978845608f * (x + 0.044715f * x * x * x))) * y;
+}
+
+// grid (slices of K = the cluster, row tiles x tiles of 128 weight rows)
+template <int TN, bool FP8>
+__global__ void __launch_bounds__(192, 2)
+gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w, const Params p) {
+  using S = Smem<TN, FP8>;
+  constexpr int KE = FP8 ? 128 : 64;                                  // elements of a K block
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const uint32_t sbase = smem_u32(smem), bar0 = sbase + S::bars;
+  auto full = [&](int s) { return bar0 + 8u * s; };
+  auto empty = [&](int s) { return bar0 + 8u * (S::stages + s); };
+  auto tfull = [&](int a) { return bar0 + 8u * (2 * S::stages + a); };
+  auto tempty = [&](int a) { return bar0 + 8u * (2 * S::stages + kAcc + a); };
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + S::bars + (2 * S::stages + 2 * kAcc) * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  float* scales = reinterpret_cast<float*>(smem + S::scales);         // [K block of the slice][row]
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int splits = gridDim.x, rank = blockIdx.x;
+  const int m_tiles = (p.M + TN - 1) / TN, mt = blockIdx.y % m_tiles, nt = blockIdx.y / m_tiles;
+  const int kb0 = (int)((int64_t)rank * p.k_blocks / splits), kb1 = (int)((int64_t)(rank + 1) * p.k_blocks / splits);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::stages; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(empty(s), 1);
+    }
+    for (int a = 0; a < kAcc; ++a) {
+      mbar_init(tfull(a), 1);
+      mbar_init(tempty(a), 4);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (p.tile_expert == nullptr && warp == 0) {
+    if (lane < kPrefetchBlocks && kb0 + lane < kb1) prefetch_2d(&tma_w, (kb0 + lane) * KE, nt * 128);
+    __syncwarp();
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  int expert = 0;
+  if (p.tile_expert != nullptr) {
+    expert = p.tile_expert[mt];
+    if (expert < 0) return;            // uniform for the cluster: nothing allocated yet
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)), "r"(S::cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_holder;
+  const int m0 = mt * TN, n0 = nt * 128;
+  const int live = min(TN, p.M - m0);
+  float acc[TN];
+  bool ok = true;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    const int wy = expert * p.N + n0;
+    for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+      const int st = i % S::stages;
+      if (!mbar_wait_warp(empty(st), ((i / S::stages) & 1) ^ 1, abort_flag)) { ok = false; break; }
+      if (lane == 0) {
+        const uint32_t dst = sbase + st * S::stage;
+        mbar_expect_tx(full(st), S::w_bytes + p.x_rows * 128);
+        tma_load_2d(dst, &tma_w, kb * KE, wy, full(st));
+        tma_load_2d(dst + S::w_bytes, &tma_x, kb * KE, m0, full(st));
+      }
+      __syncwarp();
+    }
+    if (!ok) {
+      const long long t0 = clock64();
+      while (clock64() - t0 < 20000000LL) {}          // bounded grace period for copies in flight
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    constexpr uint32_t ID = FP8 ? (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24) : idesc(false, TN);
+    for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+      const int st = i % S::stages, a = i % kAcc;
+      if (FP8 && !mbar_wait_warp(tempty(a), ((i / kAcc) & 1) ^ 1, abort_flag)) break;
+      if (!mbar_wait_warp(full(st), (i / S::stages) & 1, abort_flag)) break;
+      tc_fence_after();
+      if (lane == 0) {
+        const uint32_t w = sbase + st * S::stage, x = w + S::w_bytes;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint64_t wd = smem_desc(w + k * 32, 16, 1024), xd = smem_desc(x + k * 32, 16, 1024);
+          if constexpr (FP8) umma_fp8(tmem + a * TN, wd, xd, ID, k != 0);
+          else umma(tmem, wd, xd, ID, (i | k) != 0);
+        }
+        umma_commit(empty(st));        // the ring slot is free once these MMAs have read it
+        if (FP8) umma_commit(tfull(a));                // ... and the block's product is complete
+        else if (kb + 1 == kb1) umma_commit(tfull(0));
+      }
+      __syncwarp();
+    }
+  } else {
+    // ------------------------------------------------------------------ scale and add (warps 2..5): a thread owns a weight row
+    const int t = threadIdx.x - 64, n_kb = kb1 - kb0;
+    const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    constexpr int C = TN < 32 ? 16 : 32;
+    if constexpr (FP8) {
+      const float* ws = p.w_scale + ((int64_t)expert * p.N + n0) / 128 * p.k_blocks + kb0;
+      for (int i = t; i < n_kb * TN; i += 128) {
+        const int r = i / n_kb, k = i - r * n_kb;
+        scales[k * TN + r] = r < live ? p.a_scale[(int64_t)(m0 + r) * p.k_blocks + kb0 + k] * ws[k] : 0.f;
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[j] = 0.f;
+      for (int i = 0; i < n_kb; ++i) {
+        const int a = i % kAcc;
+        ok = ok && mbar_wait(tfull(a), (i / kAcc) & 1, abort_flag);
+        __syncwarp();
+        tc_fence_after();
+        uint32_t r[TN];
+#pragma unroll
+        for (int j = 0; j < TN; j += C) {
+          if constexpr (C == 16) tmem_ld16(at + a * TN + j, r + j);
+          else tmem_ld32(at + a * TN + j, r + j);
+        }
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tempty(a));        // handed back before the arithmetic
+        const float4* sc = reinterpret_cast<const float4*>(scales + i * TN);
+#pragma unroll
+        for (int j = 0; j < TN; j += 4) {
+          const float4 f = sc[j >> 2];
+          acc[j] = fmaf(__uint_as_float(r[j]), f.x, acc[j]);
+          acc[j + 1] = fmaf(__uint_as_float(r[j + 1]), f.y, acc[j + 1]);
+          acc[j + 2] = fmaf(__uint_as_float(r[j + 2]), f.z, acc[j + 2]);
+          acc[j + 3] = fmaf(__uint_as_float(r[j + 3]), f.w, acc[j + 3]);
+        }
+      }
+    } else {
+      ok = mbar_wait(tfull(0), 0, abort_flag);
+      __syncwarp();
+      tc_fence_after();
+      uint32_t r[TN];
+#pragma unroll
+      for (int j = 0; j < TN; j += C) {
+        if constexpr (C == 16) tmem_ld16(at + j, r + j);
+        else tmem_ld32(at + j, r + j);
+      }
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[j] = __uint_as_float(r[j]);
+    }
+  }
+  const int row = (warp & 3) * 32 + lane;             // warps 2..5: tensor memory lane = weight row of the tile
+  const bool stores = warp >= 2 && n0 + row < p.N;
+  const float bias = !FP8 && stores && p.bias != nullptr ? __bfloat162float(p.bias[n0 + row]) : 0.f;
+  float* red = reinterpret_cast<float*>(smem);        // [row of A][weight row]: every copy of the ring has been consumed
+  float* fin = splits > 1 ? red + TN * 128 : red;     // what the activation reads
+  if (splits == 1) {
+    if (!FP8 && p.act != 0) {
+      if (warp >= 2) {
+#pragma unroll
+        for (int j = 0; j < TN; ++j) fin[j * 128 + row] = acc[j];
+      }
+    } else if (stores && ok) {
+      bf16* dst = p.c + (int64_t)m0 * p.ldc + n0 + row;
+#pragma unroll
+      for (int j = 0; j < TN; ++j)
+        if (j < live) dst[j * p.ldc] = __float2bfloat16(acc[j] + bias);
+    }
+  } else {
+    if (warp >= 2)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) red[j * 128 + row] = acc[j];
+    __syncwarp();
+    cluster_sync();
+    if (warp >= 2)
+      for (int j = rank; j < live; j += splits) {
+        const uint32_t at = sbase + (uint32_t)(j * 128 + row) * 4;
+        float v[kMaxSplit], sum = 0.f;
+#pragma unroll
+        for (int s = 0; s < kMaxSplit; ++s) v[s] = s < splits ? ld_cluster(at, s) : 0.f;
+#pragma unroll
+        for (int s = 0; s < kMaxSplit; ++s) sum += v[s];
+        if (!FP8 && p.act != 0) fin[j * 128 + row] = sum;
+        else if (stores && ok) p.c[(int64_t)(m0 + j) * p.ldc + n0 + row] = __float2bfloat16(sum + bias);
+      }
+    __syncwarp();
+  }
+  if (!FP8 && p.act != 0 && warp >= 2) {              // N a multiple of 128
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    const int f = row & 63;
+    const auto rounded = [](float x) { return __bfloat162float(__float2bfloat16(x)); };   // as the two-launch form stores them
+    if (ok)
+      for (int j = rank + splits * (row >> 6); j < live; j += 2 * splits)
+        p.c[(int64_t)(m0 + j) * p.ldc + nt * 64 + f] =
+            __float2bfloat16(gated(rounded(fin[j * 128 + f]), rounded(fin[j * 128 + 64 + f]), p.act, p.limit, p.alpha));
+  }
+  if (splits > 1) cluster_sync();                     // nobody leaves while its sums are being read
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag && p.err != nullptr) atomicExch(p.err, 1);
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::cols));
+  }
+}
+
+static int* g_err[64] = {};
+
+// [rows, cols] with row stride ld elements; box = [box_rows, 128 bytes], 128-byte swizzle
+static bool make_map_of(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows, bool fp8) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * (fp8 ? 1 : 2)};
+  cuuint32_t box[2] = {fp8 ? 128u : 64u, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides,
+            box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// How many CTAs cut K: an SM works through ceil(tiles x s / 148) slices of ceil(k_blocks / s) blocks, each with a start and
+// an end worth about three blocks of its bandwidth; meeting costs about two more.
+static int choose_split(int tiles, int k_blocks) {
+  int best = 1;
+  double cost = 1e30;
+  for (int s = 1; s <= kMaxSplit && s <= k_blocks; ++s) {
+    const int waves = (tiles * s + 147) / 148;
+    const double c = waves * ((k_blocks + s - 1) / s + 3.0) + (s > 1 ? 2.0 : 0.0);
+    if (c < cost - 1e-9) { cost = c; best = s; }
+  }
+  return best;
+}
+
+template <int TN, bool FP8>
+static int launch(const void* a, const void* w, const Params& p, int K, int64_t lda, int64_t ldw, int n_experts, int splits,
+                  int dev, cudaStream_t s) {
+  using S = Smem<TN, FP8>;
+  static std::atomic<int> attr_bytes[64] = {};
+  const int per = (p.k_blocks + splits - 1) / splits, smem = S::total(per);
+  if (smem > 232448) return (int)cudaErrorInvalidValue;
+  if (attr_bytes[dev & 63].load(std::memory_order_acquire) < smem) {
+    // once and for all sizes: a kernel may use what its launch asks for, up to this
+    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<TN, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    if (e != cudaSuccess) return (int)e;
+    attr_bytes[dev & 63].store(232448, std::memory_order_release);
+  }
+  CUtensorMap tx, tw;
+  if (!make_map_of(&tx, a, p.M, K, lda, p.x_rows, FP8) || !make_map_of(&tw, w, (int64_t)p.N * n_experts, K, ldw, 128, FP8))
+    return (int)cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(splits, (unsigned)(((p.M + TN - 1) / TN) * ((p.N + 127) / 128)));
+  cfg.blockDim = dim3(192);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = splits;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_few_kernel<TN, FP8>, tx, tw, p);
+  return e != cudaSuccess ? (int)e : XLLM_LAUNCH_CHECK();
+}
+
+// tile: rows of A at a time.  Grouped: every tile belongs to one expert, M a multiple of it.
+template <bool FP8>
+static int run(const void* a, const void* w, Params p, int n_experts, int tile, int K, int64_t lda, int64_t ldw, cudaStream_t s) {
+  constexpr int KE = FP8 ? 128 : 64;
+  if ((tile != 16 && tile != 32 && tile != 64) || n_experts < 1 || (p.tile_expert != nullptr && (p.M % tile || p.N % 128)) ||
+      (((uintptr_t)a | (uintptr_t)w | (uintptr_t)p.c) & 15))
+    return (int)cudaErrorInvalidValue;
+  p.k_blocks = (K + KE - 1) / KE;
+  p.x_rows = p.M >= tile ? tile : ((p.M + 7) & ~7);
+  const int64_t tiles = (int64_t)((p.M + tile - 1) / tile) * ((p.N + 127) / 128);
+  if (tiles > 65535) return (int)cudaErrorInvalidValue;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (g_err[dev & 63] == nullptr) {
+    if (cudaMalloc(&g_err[dev & 63], sizeof(int)) != cudaSuccess) return (int)cudaErrorMemoryAllocation;
+    cudaMemset(g_err[dev & 63], 0, sizeof(int));
+  }
+  p.err = g_err[dev & 63];
+  // a grouped launch holds tiles of experts nobody chose: how many are live is not known here, and there are many
+  const int splits = p.tile_expert != nullptr ? 1 : choose_split((int)tiles, p.k_blocks);
+  if (tile == 16) return launch<16, FP8>(a, w, p, K, lda, ldw, n_experts, splits, dev, s);
+  if (tile == 32) return launch<32, FP8>(a, w, p, K, lda, ldw, n_experts, splits, dev, s);
+  return launch<64, FP8>(a, w, p, K, lda, ldw, n_experts, splits, dev, s);
+}
+
+static Params make_params(void* c, int64_t ldc, int M, int N, const void* tile_expert) {
+  Params p{};
+  p.c = (bf16*)c; p.ldc = ldc; p.M = M; p.N = N; p.tile_expert = (const int32_t*)tile_expert;
+  return p;
+}
+
+}  // namespace few
+}  // namespace xllm
+
+// C[M, N] = A[M, K] W[N, K]^T (+ bias[N]) for up to 64 rows.  K, N, lda, ldw % 8 == 0, 16-byte aligned bases.
+XLLM_API int xllm_gemm_bf16_few(const void* a, const void* w, void* c, const void* bias, int M, int N, int K, int64_t lda,
+                                int64_t ldw, int64_t ldc, void* stream) {
+  using namespace xllm::few;
+  if (M == 0 || N == 0) return 0;
+  if (M > 64 || K <= 0 || K % 8 || N % 8 || lda % 8 || ldw % 8) return (int)cudaErrorInvalidValue;
+  Params p = make_params(c, ldc, M, N, nullptr);
+  p.bias = (const xllm::bf16*)bias;
+  return run<false>(a, w, p, 1, M <= 16 ? 16 : (M <= 32 ? 32 : 64), K, lda, ldw, (cudaStream_t)stream);
+}
+
+// The same for xllm_gemm_bf16_act_mul's contract: N rows of interleaved gate and up, N % 128 == 0, C [M, N / 2], act 1 .. 4.
+XLLM_API int xllm_gemm_bf16_act_mul_few(const void* a, const void* w, void* c, int M, int N, int K, int64_t lda, int64_t ldw,
+                                        int64_t ldc, int act, float limit, float alpha, void* stream) {
+  using namespace xllm::few;
+  if (M == 0 || N == 0) return 0;
+  if (M > 64 || K <= 0 || K % 8 || N % 128 || lda % 8 || ldw % 8 || act < 1 || act > 4) return (int)cudaErrorInvalidValue;
+  Params p = make_params(c, ldc, M, N, nullptr);
+  p.act = act; p.limit = limit; p.alpha = alpha;
+  return run<false>(a, w, p, 1, M <= 16 ? 16 : (M <= 32 ? 32 : 64), K, lda, ldw, (cudaStream_t)stream);
+}
+
+// xllm_gemm_bf16_grouped and (act != 0) xllm_gemm_bf16_grouped_act_mul over tiles of `tile` rows (16, 32, 64); N % 128 == 0.
+XLLM_API int xllm_gemm_bf16_grouped_few(const void* a, const void* w, void* c, const void* tile_expert, int tile, int M, int N,
+                                        int K, int n_experts, int64_t lda, int64_t ldc, int act, float limit, float alpha,
+                                        void* stream) {
+  using namespace xllm::few;
+  if (M == 0 || N == 0) return 0;
+  if (tile_expert == nullptr || K <= 0 || K % 8 || lda % 8 || act < 0 || act > 4) return (int)cudaErrorInvalidValue;
+  Params p = make_params(c, ldc, M, N, tile_expert);
+  p.act = act; p.limit = limit; p.alpha = alpha;
+  return run<false>(a, w, p, n_experts, tile, K, lda, K, (cudaStream_t)stream);
+}
+
+// The contracts of xllm_gemm_fp8_block and (tile_expert not null) xllm_gemm_fp8_block_grouped, `tile` rows of A (16, 32 or 64)
+// at a time.
+XLLM_API int xllm_gemm_fp8_few(const void* a, const void* w, void* c, const void* a_scale, const void* w_scale,
+                               const void* tile_expert, int n_experts, int tile, int M, int N, int K, int64_t lda, int64_t ldw,
+                               int64_t ldc, void* stream) {
+  using namespace xllm::few;
+  if (M == 0 || N == 0) return 0;
+  if (K % 128 || K <= 0 || N % 8 || lda % 16 || ldw % 16) return (int)cudaErrorInvalidValue;
+  Params p = make_params(c, ldc, M, N, tile_expert);
+  p.a_scale = (const float*)a_scale; p.w_scale = (const float*)w_scale;
+  return run<true>(a, w, p, n_experts, tile, K, lda, ldw, (cudaStream_t)stream);
+}
+
+// 0 = no bounded wait expired in these kernels on this device since the last call.
+XLLM_API int xllm_gemm_few_error_status() {
+  using namespace xllm::few;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (g_err[dev & 63] == nullptr) return 0;
+  int v = 0;
+  cudaMemcpy(&v, g_err[dev & 63], sizeof(int), cudaMemcpyDeviceToHost);
+  if (v != 0) cudaMemset(g_err[dev & 63], 0, sizeof(int));
+  return v;
+}

@@ -164,37 +164,55 @@ __global__ void __launch_bounds__(128) moe_route_kernel(RouteParams p) {
   }
 }
 
-// offsets[e] = first row of expert e in the permuted buffer (multiple of 128); tile_expert[i] =
-// expert of row tile i (or -1); counts are cleared for the next call; meta[0] = rows used.
-__global__ void moe_offsets_kernel(int32_t* counts, int32_t* offsets, int32_t* tile_expert, int32_t* meta, int E,
-                                   int max_tiles, int expert_begin) {
+// offsets[e] = first row of expert e in the permuted buffer (multiple of `tile`); tile_expert[i] =
+// expert of row tile i (or -1); counts are cleared for the next call; meta[0] = rows used.  One block: the counts are
+// loaded side by side and summed by a warp (one thread walking them took 5.5 us for 128 experts, a load's latency each).
+__global__ void __launch_bounds__(256) moe_offsets_kernel(int32_t* counts, int32_t* offsets, int32_t* tile_expert, int32_t* meta,
+                                                          int E, int max_tiles, int expert_begin, int tile) {
   __shared__ int s_off[kMaxExperts + 1];
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < E; ++e) {
-      s_off[e] = acc;
-      acc += (counts[e] + kMoeTile - 1) / kMoeTile * kMoeTile;
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    s_off[e + 1] = (counts[e] + tile - 1) / tile * tile;
+    counts[e] = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    int base = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + threadIdx.x;
+      int v = e < E ? s_off[e + 1] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (threadIdx.x >= o) v += u;
+      }
+      if (e < E) s_off[e + 1] = base + v;
+      base += __shfl_sync(0xffffffffu, v, 31);
     }
-    s_off[E] = acc;
-    meta[0] = acc;
+    if (threadIdx.x == 0) {
+      s_off[0] = 0;
+      meta[0] = base;
+    }
   }
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     offsets[e] = s_off[e];
-    const int t0 = s_off[e] / kMoeTile, t1 = s_off[e + 1] / kMoeTile;
+    const int t0 = s_off[e] / tile, t1 = s_off[e + 1] / tile;
     for (int i = t0; i < t1 && i < max_tiles; ++i) tile_expert[i] = e - expert_begin;  // index into the local weights
   }
-  for (int i = s_off[E] / kMoeTile + threadIdx.x; i < max_tiles; i += blockDim.x) tile_expert[i] = -1;
-  __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
+  for (int i = s_off[E] / tile + threadIdx.x; i < max_tiles; i += blockDim.x) tile_expert[i] = -1;
 }
 
-// xp[row(t,k), :] = x[t, :]; rows[t,k] = offsets[e] + slot (or -1 for non-local experts); a row is n_vec vectors of V
+// xp[row(t,k), :] = x[t, :] (and a quantised row's scales beside it); rows[t,k] = offsets[e] + slot (or -1 for non-local experts); a row is n_vec vectors of V
 template <typename V>
 __global__ void __launch_bounds__(256)
 moe_permute_kernel(V* __restrict__ xp, int32_t* __restrict__ rows, const V* __restrict__ x, const int32_t* __restrict__ topk_ids,
-                   const int32_t* __restrict__ slot, const int32_t* __restrict__ offsets, int T, int K, int n_vec) {
+                   const int32_t* __restrict__ slot, const int32_t* __restrict__ offsets, int T, int K, int n_vec,
+                   float* __restrict__ sp, const float* __restrict__ scales, int n_scales) {
   const int pair = blockIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = pair / K;
   const int s = slot[pair];
   int row = -1;
@@ -204,6 +222,7 @@ moe_permute_kernel(V* __restrict__ xp, int32_t* __restrict__ rows, const V* __re
   const V* src = x + (int64_t)t * n_vec;
   V* dst = xp + (int64_t)row * n_vec;
   for (int v = threadIdx.x; v < n_vec; v += blockDim.x) dst[v] = src[v];
+  for (int v = threadIdx.x; v < n_scales; v += blockDim.x) sp[(int64_t)row * n_scales + v] = scales[(int64_t)t * n_scales + v];
 }
 
 template <typename T_, int V>
@@ -211,6 +230,8 @@ __global__ void __launch_bounds__(256)
 moe_finalize_kernel(T_* __restrict__ out, const T_* __restrict__ y, int64_t y_ld, const int32_t* __restrict__ rows,
                     const float* __restrict__ w, const T_* __restrict__ shared_out, int T, int K, int H) {
   const int t = blockIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
   for (int v = threadIdx.x; v < H / V; v += blockDim.x) {
     float acc[V];
     if (shared_out) load_f32<V>(shared_out + (int64_t)t * H + v * V, acc);
@@ -300,28 +321,45 @@ XLLM_API int xllm_moe_route(const void* logits, int logits_fp32, const void* bia
                            renorm, scale, expert_begin, expert_end, stream);
 }
 
+// `tile`: rows of a tile, none of which two experts share
+XLLM_API int xllm_moe_offsets_tile(void* counts, void* offsets, void* tile_expert, void* meta, int E, int max_tiles,
+                                   int expert_begin, int tile, void* stream) {
+  using namespace xllm;
+  if (E <= 0 || E > kMaxExperts || tile <= 0) return (int)cudaErrorInvalidValue;
+  launch_pdl(moe_offsets_kernel, dim3(1), dim3(256), 0, (cudaStream_t)stream, (int32_t*)counts, (int32_t*)offsets,
+             (int32_t*)tile_expert, (int32_t*)meta, E, max_tiles, expert_begin, tile);
+  return XLLM_LAUNCH_CHECK();
+}
 XLLM_API int xllm_moe_offsets(void* counts, void* offsets, void* tile_expert, void* meta, int E, int max_tiles,
                               int expert_begin, void* stream) {
+  return xllm_moe_offsets_tile(counts, offsets, tile_expert, meta, E, max_tiles, expert_begin, xllm::kMoeTile, stream);
+}
+
+static int moe_permute(void* xp, void* rows, const void* x, const void* topk_ids, const void* slot, const void* offsets, int T,
+                       int K, int bytes, void* sp, const void* scales, int n_scales, void* stream) {
   using namespace xllm;
-  moe_offsets_kernel<<<1, 256, 0, (cudaStream_t)stream>>>((int32_t*)counts, (int32_t*)offsets, (int32_t*)tile_expert,
-                                                         (int32_t*)meta, E, max_tiles, expert_begin);
+  if (T == 0) return 0;
+  const auto run = [&](auto tag, int n_vec) {
+    using V = decltype(tag);
+    launch_pdl(moe_permute_kernel<V>, dim3(T * K), dim3(256), 0, (cudaStream_t)stream, (V*)xp, (int32_t*)rows, (const V*)x,
+               (const int32_t*)topk_ids, (const int32_t*)slot, (const int32_t*)offsets, T, K, n_vec, (float*)sp,
+               (const float*)scales, n_scales);
+  };
+  if (bytes % 16 == 0 && (((uintptr_t)xp | (uintptr_t)x) & 15) == 0) run(uint4(), bytes / 16);
+  else run((unsigned short)0, bytes / 2);
   return XLLM_LAUNCH_CHECK();
 }
 
 // dtype of the entry points below: 0 bf16, 1 fp32.
 XLLM_API int xllm_moe_permute(void* xp, void* rows, const void* x, const void* topk_ids, const void* slot,
                               const void* offsets, int T, int K, int H, int dtype, void* stream) {
-  using namespace xllm;
-  if (T == 0) return 0;
-  const auto run = [&](auto tag, int n_vec) {
-    using V = decltype(tag);
-    moe_permute_kernel<V><<<T * K, 256, 0, (cudaStream_t)stream>>>((V*)xp, (int32_t*)rows, (const V*)x, (const int32_t*)topk_ids,
-                                                                  (const int32_t*)slot, (const int32_t*)offsets, T, K, n_vec);
-  };
-  const int bytes = H * (dtype == 0 ? 2 : 4);
-  if (bytes % 16 == 0 && (((uintptr_t)xp | (uintptr_t)x) & 15) == 0) run(uint4(), bytes / 16);
-  else run((unsigned short)0, bytes / 2);
-  return XLLM_LAUNCH_CHECK();
+  return moe_permute(xp, rows, x, topk_ids, slot, offsets, T, K, H * (dtype == 0 ? 2 : 4), nullptr, nullptr, 0, stream);
+}
+
+// Rows of H e4m3 values (H even) and their n_scales fp32 scales.
+XLLM_API int xllm_moe_permute_fp8(void* xp, void* sp, void* rows, const void* x, const void* scales, const void* topk_ids,
+                                  const void* slot, const void* offsets, int T, int K, int H, int n_scales, void* stream) {
+  return moe_permute(xp, rows, x, topk_ids, slot, offsets, T, K, H, sp, scales, n_scales, stream);
 }
 
 // y: rows of y_ld elements, of which the first H count
@@ -332,8 +370,8 @@ XLLM_API int xllm_moe_finalize(void* out, const void* y, int64_t y_ld, const voi
   const bool v8 = H % 8 == 0 && y_ld % 8 == 0 && (((uintptr_t)out | (uintptr_t)y | (uintptr_t)shared_out) & 15) == 0;
   const auto run = [&](auto tag, auto kernel) {
     using E = decltype(tag);
-    kernel<<<T, 256, 0, (cudaStream_t)stream>>>((E*)out, (const E*)y, y_ld, (const int32_t*)rows, (const float*)w,
-                                                (const E*)shared_out, T, K, H);
+    launch_pdl(kernel, dim3(T), dim3(256), 0, (cudaStream_t)stream, (E*)out, (const E*)y, y_ld, (const int32_t*)rows,
+               (const float*)w, (const E*)shared_out, T, K, H);
   };
   if (dtype == 0) {
     if (v8) run(bf16(), moe_finalize_kernel<bf16, 8>);

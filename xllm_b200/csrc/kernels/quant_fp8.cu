@@ -62,6 +62,8 @@ quant_group128_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, const
   const int groups = H >> 7;
   const int64_t g = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 4);  // 16 groups per CTA
   const int l = threadIdx.x & 15;
+  pdl_wait();
+  pdl_launch_dependents();
   const bool active = g < T * groups;
   const int64_t row = active ? g / groups : 0;
   const int gi = active ? (int)(g - row * groups) : 0;
@@ -85,6 +87,54 @@ quant_group128_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, const
 #pragma unroll
   for (int j = 0; j < 8; ++j) ob[j] = to_e4m3(f[j] * inv);
   reinterpret_cast<uint2*>(q + row * (int64_t)H + gi * 128)[l] = o;
+}
+
+// Gated activation of x [rows, 2 d] = gate | up, rounded to bf16 as act_and_mul_kernel writes it, and its quantisation by groups
+// of 128: one pass instead of two (922 prompt rows on 32 experts, 11.5 thousand permuted rows of 2 x 2048: 112 + 21 us).
+// Rows of tiles that no expert has (tile_expert < 0) are left.
+__global__ void __launch_bounds__(256)
+act_quant_group128_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, const bf16* __restrict__ x, int64_t rows, int d,
+                          const int32_t* __restrict__ tile_expert, int tile, int act, float limit, float alpha) {
+  const int groups = d >> 7;
+  const int64_t g = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 4);
+  const int l = threadIdx.x & 15;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int64_t row = g / groups;
+  const int gi = (int)(g - row * groups);
+  const bool active = row < rows && (tile_expert == nullptr || tile_expert[row / tile] >= 0);
+  float f[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = 0.f;
+  if (active) {
+    const bf16x8* src = reinterpret_cast<const bf16x8*>(x + row * 2 * d) + gi * 16 + l;
+    float a[8], b[8];
+    unpack8(src[0], a);
+    unpack8(src[d >> 3], b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float y;
+      if (act == 3) y = clamped_glu(a[j], b[j], limit, alpha);
+      else if (act == 0) y = a[j] / (1.f + __expf(-a[j])) * b[j];
+      else if (act == 1) y = 0.5f * a[j] * (1.f + erff(a[j] * 0.70710678f)) * b[j];
+      else y = 0.5f * a[j] * (1.f + tanhf(0.7978845608f * (a[j] + 0.044715f * a[j] * a[j] * a[j]))) * b[j];
+      f[j] = __bfloat162float(__float2bfloat16(y));
+    }
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(f[j]));
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (!active) return;
+  const float s = fmaxf(amax, 1e-10f) / 448.f;
+  if (l == 0) scales[row * groups + gi] = s;
+  const float inv = 1.f / s;
+  uint2 o;
+  uint8_t* ob = reinterpret_cast<uint8_t*>(&o);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) ob[j] = to_e4m3(f[j] * inv);
+  reinterpret_cast<uint2*>(q + row * (int64_t)d + gi * 128)[l] = o;
 }
 
 // w[n, k] = q[n, k] * scales[n / 128, k / 128]
@@ -124,8 +174,22 @@ XLLM_API int xllm_quant_fp8_group128(void* q, void* scales, const void* x, int64
   if (T == 0) return 0;
   if (H % 128) return (int)cudaErrorInvalidValue;
   const int64_t groups = T * (H / 128);
-  quant_group128_kernel<<<(unsigned)((groups + 15) / 16), 256, 0, (cudaStream_t)stream>>>(
-      (uint8_t*)q, (float*)scales, (const bf16*)x, T, H, x_stride);
+  launch_pdl(quant_group128_kernel, dim3((unsigned)((groups + 15) / 16)), dim3(256), 0, (cudaStream_t)stream, (uint8_t*)q,
+             (float*)scales, (const bf16*)x, T, H, x_stride);
+  return XLLM_LAUNCH_CHECK();
+}
+
+// q [rows, d] e4m3, scales [rows, d / 128] of the gated activation of x [rows, 2 d] (act: see xllm_act_and_mul).  tile_expert
+// (or null): rows of a tile of `tile` whose entry is negative are skipped.  d % 128 == 0, x 16-byte aligned.
+XLLM_API int xllm_act_quant_fp8_group128(void* q, void* scales, const void* x, int64_t rows, int d, const void* tile_expert,
+                                         int tile, int act, float limit, float alpha, void* stream) {
+  using namespace xllm;
+  if (rows == 0) return 0;
+  if (d <= 0 || d % 128 || act < 0 || act > 3 || (tile_expert != nullptr && tile <= 0) || (((uintptr_t)x) & 15))
+    return (int)cudaErrorInvalidValue;
+  const int64_t groups = rows * (d / 128);
+  launch_pdl(act_quant_group128_kernel, dim3((unsigned)((groups + 15) / 16)), dim3(256), 0, (cudaStream_t)stream, (uint8_t*)q,
+             (float*)scales, (const bf16*)x, rows, d, (const int32_t*)tile_expert, tile, act, limit, alpha);
   return XLLM_LAUNCH_CHECK();
 }
 

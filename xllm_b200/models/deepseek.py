@@ -221,7 +221,8 @@ class MLAAttention(Module):
         w = self.kv_b_proj.weight.view(nh, self.nope + self.vd, L)
         w_uk, w_uv = w[:, :self.nope], w[:, self.nope:]        # [nh, nope, L], [nh, vd, L]
         q_cat = torch.empty((T, nh, L + r), dtype=x.dtype, device=x.device)
-        q_cat[..., :L] = torch.einsum("thn,hnl->thl", q[..., :self.nope], w_uk)
+        # the products land in their places: no copy of them in another order
+        torch.bmm(q[..., :self.nope].transpose(0, 1), w_uk, out=q_cat[..., :L].transpose(0, 1))
         mla_ops.cache_write(kv_a, self.kv_a_layernorm.weight, self.kv_a_layernorm.eps, self.rope.cos_sin, positions,
                             meta.slots, cache, q[..., self.nope:], q_cat)
         o_lat = torch.empty((T, nh, L), dtype=x.dtype, device=x.device)
@@ -241,8 +242,9 @@ class MLAAttention(Module):
             seq = torch.bucketize(tok, meta.cu_q[nd + 1:].contiguous(), right=True).clamp_(max=meta.n_prefill - 1)
             mla_ops.decode(q_cat[nd:], cache, meta.block_table, self.scale, positions=positions[nd:],
                            bt_rows=(seq + nd).to(torch.int32), out=o_lat[nd:], latent=L)
-        out = torch.einsum("thl,hvl->thv", o_lat, w_uv)
-        return self.o_proj(out.reshape(T, nh * self.vd))
+        out = torch.empty((T, nh, self.vd), dtype=x.dtype, device=x.device)
+        torch.bmm(o_lat.transpose(0, 1), w_uv.transpose(1, 2), out=out.transpose(0, 1))
+        return self.o_proj(out.view(T, nh * self.vd))
 
     def _sparse_attend(self, q_cat, cache, meta, positions, sel, n_sel, o_lat):
         """Attention of every query row over ITS selected context tokens: their latent rows are gathered

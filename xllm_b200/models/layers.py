@@ -594,7 +594,8 @@ class DenseMLP(Module):
         gu = self.gate_up
         if gu.interleaved:
             from ..ops import gemm, gemm_tcgen05
-            if (x.is_cuda and x.dim() == 2 and x.shape[0] > 512 and gemm.gemm_mode() != "cublas" and gu.weight.shape[0] % 256 == 0
+            # (in between, narrower tiles and a kernel of its own for the activation are quicker)
+            if (x.is_cuda and x.dim() == 2 and (x.shape[0] > 512 or gemm_tcgen05.few_rows(x.shape[0], gu.weight.shape[0])) and gemm.gemm_mode() != "cublas" and gu.weight.shape[0] % 256 == 0
                     and gemm_tcgen05.supported(x, gu.weight)):
                 return gemm_tcgen05.gemm_act_mul(x, gu.weight, self.act)
             y = gu(x)

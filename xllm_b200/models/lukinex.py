@@ -129,7 +129,7 @@ class LukinexCausalLM(Module):
     supports_graph = True
     supports_prefill_graph = True
     # the kernel sources a process that runs nothing but this model needs
-    kernel_sources = ("gemm_tcgen05", "activation", "attn_decode", "attn_prefill", "attn_prefill_tc", "attn_generic",
+    kernel_sources = ("gemm_tcgen05", "gemm_few", "activation", "attn_decode", "attn_prefill", "attn_prefill_tc", "attn_generic",
                       "linear_attn", "head_norm", "mla", "proj_f32", "moe", "residual", "rope_norm_kv", "misc", "sampling")
     fused_tp = False
 

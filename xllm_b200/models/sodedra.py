@@ -103,7 +103,7 @@ class SodedraCausalLM(Module):
     supports_graph = True
     supports_prefill_graph = True
     # the kernel sources a process that runs nothing but this model needs
-    kernel_sources = ("gemm_tcgen05", "activation", "attn_decode", "attn_prefill", "attn_prefill_tc", "attn_generic",
+    kernel_sources = ("gemm_tcgen05", "gemm_few", "activation", "attn_decode", "attn_prefill", "attn_prefill_tc", "attn_generic",
                       "delta_rule", "mlstm", "head_norm", "proj_f32", "moe", "residual", "rope_norm_kv", "misc", "sampling")
     fused_tp = False
 

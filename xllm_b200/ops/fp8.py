@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from ._lib import I, L, P, check, ptr, stream
+from ._lib import F, I, L, P, check, ptr, stream
 
 _lib.register_signature("xllm_gemm_fp8", [P, P, P, P, P, P, I, I, I, I, I, L, L, L, P])
 _lib.register_signature("xllm_quant_fp8_per_token", [P, P, P, P, L, I, L, P])
@@ -19,7 +19,11 @@ _lib.register_signature("xllm_dequant_fp8_block128", [P, P, P, L, I, P])
 _lib.register_signature("xllm_gemm_fp8_block", [P, P, P, P, P, I, I, I, L, L, L, P])
 _lib.register_signature("xllm_gemm_fp8_block_grouped", [P, P, P, P, P, P, I, I, I, I, L, L, L, P])
 
+_lib.register_signature("xllm_gemm_fp8_few", [P, P, P, P, P, P, I, I, I, I, I, L, L, L, P])
+_lib.register_signature("xllm_act_quant_fp8_group128", [P, P, P, L, I, P, I, I, F, F, P])
+
 FP8 = torch.float8_e4m3fn
+FEW_ROWS = 64        # most rows of the product whose tile is 128 weight rows (csrc/kernels/gemm_few.cu)
 FP8_MAX = 448.0
 
 
@@ -159,6 +163,14 @@ def block_scaled_mm(a_q, a_scale, w_q, w_scale, out=None):
     assert w_scale.dtype == torch.float32 and w_scale.is_contiguous() and w_scale.shape == ((N + 127) // 128, K // 128)
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=a_q.device)
+    # few rows: bound by the weights' way from HBM; from 65 rows on a tile of 128 rows of a_q wastes less than two passes
+    if 0 < M <= FEW_ROWS:
+        check(_lib.load().xllm_gemm_fp8_few(ptr(a_q), ptr(w_q), ptr(out), ptr(a_scale), ptr(w_scale), None, 1,
+                                            16 if M <= 16 else 32 if M <= 32 else 64, M, N, K, a_q.stride(0), w_q.stride(0),
+                                            out.stride(0), stream()), "gemm_fp8_few")
+        from . import _count
+        _count()
+        return out
     check(_lib.load().xllm_gemm_fp8_block(ptr(a_q), ptr(w_q), ptr(out), ptr(a_scale), ptr(w_scale), M, N, K,
                                           a_q.stride(0), w_q.stride(0), out.stride(0), stream()), "gemm_fp8_block")
     from . import _count
@@ -166,13 +178,37 @@ def block_scaled_mm(a_q, a_scale, w_q, w_scale, out=None):
     return out
 
 
-def block_scaled_mm_grouped(a_q, a_scale, w_q, w_scale, tile_expert, out):
-    """Grouped form: rows of a_q are sorted by expert in 128-row tiles, tile_expert [rows / 128] int32
+def act_quant_group128(x, act, tile_expert=None, tile=128):
+    """quant_group128 of the gated activation of x [rows, 2 d] = gate | up (bf16, contiguous); rows of tiles with a negative
+    entry in tile_expert are left out."""
+    from . import glu
+    rows, d = x.shape[0], x.shape[1] // 2
+    if not x.is_cuda:
+        return quant_group128_ref(glu.apply(x[:, :d].float(), x[:, d:].float(), act).to(x.dtype))
+    assert x.dtype == torch.bfloat16 and x.is_contiguous()
+    q = torch.empty(rows, d, dtype=FP8, device=x.device)
+    s = torch.empty(rows, d // 128, dtype=torch.float32, device=x.device)
+    code, limit, alpha = glu.code(act)
+    check(_lib.load().xllm_act_quant_fp8_group128(ptr(q), ptr(s), ptr(x), rows, d, ptr(tile_expert), tile, code, limit, alpha,
+                                                  stream()), "act_quant_fp8_group128")
+    from . import _count
+    _count()
+    return q, s
+
+
+def block_scaled_mm_grouped(a_q, a_scale, w_q, w_scale, tile_expert, out, tile=128):
+    """Grouped form: rows of a_q are sorted by expert in tiles of `tile` rows (16, 32, 64 or 128), tile_expert [rows / tile] int32
     (-1: unused); w_q [E, N, K] e4m3, w_scale [E, N / 128, K / 128]; out [rows, N] bf16."""
     E, N, K = w_q.shape
     rows = a_q.shape[0]
     assert a_q.dtype == FP8 and w_q.dtype == FP8 and w_q.is_contiguous() and w_scale.is_contiguous()
     assert a_scale.shape == (rows, K // 128) and a_scale.is_contiguous() and N % 128 == 0
+    if tile != 128:
+        check(_lib.load().xllm_gemm_fp8_few(ptr(a_q), ptr(w_q), ptr(out), ptr(a_scale), ptr(w_scale), ptr(tile_expert), E, tile,
+                                            rows, N, K, a_q.stride(0), K, out.stride(0), stream()), "gemm_fp8_few")
+        from . import _count
+        _count()
+        return out
     check(_lib.load().xllm_gemm_fp8_block_grouped(ptr(a_q), ptr(w_q), ptr(out), ptr(a_scale), ptr(w_scale),
                                                   ptr(tile_expert), E, rows, N, K, a_q.stride(0), K, out.stride(0),
                                                   stream()), "gemm_fp8_block_grouped")

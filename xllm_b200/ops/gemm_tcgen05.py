@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes
+import os
 
 import torch
 
@@ -57,6 +58,23 @@ def unpack_weight(pw: PackedWeight):
     return pw.data.view(N // 64, K // 64, 64, 64).permute(0, 2, 1, 3).reshape(N, K)
 
 
+# Up to this many rows a product is the weights' way from HBM and runs with the weights as the rows of the tile
+# (csrc/kernels/gemm_few.cu); a larger one fills tiles of 128 token rows.  XLLM_GEMM_MAX_CTAS caps the grid of the other kernel.
+FEW_ROWS = 64
+_ALL_SMS = "XLLM_GEMM_MAX_CTAS" not in os.environ
+
+
+def few_rows(M, N):
+    """Beyond 32 rows the tokens' way to each of many tiles of 128 weight rows counts (64 x 24576 x 4096: 51 us against 44 us in
+    tiles of 192); that kernel keeps the products whose tiles alone would leave SMs idle (64 x 4096 x 12288: 26 us against
+    28, 64 x 12288 x 2048 gated: 14 us against 26 and the activation's own)."""
+    return _ALL_SMS and (0 < M <= 32 or (M <= FEW_ROWS and N <= 148 * 128))
+
+
+_lib.register_signature("xllm_gemm_bf16_few", [P, P, P, P, I, I, I, L, L, L, P])
+_lib.register_signature("xllm_gemm_bf16_act_mul_few", [P, P, P, I, I, I, L, L, L, I, F, F, P])
+
+
 def gemm_nt(x, w, bias=None, out=None, tile_n: int = 0, pair: int = -1, split_k: int = 0):
     """y[..., N] = x[..., K] @ w[N, K]^T (+ bias).  `w` is a tensor or a PackedWeight."""
     packed = isinstance(w, PackedWeight)
@@ -77,6 +95,11 @@ def gemm_nt(x, w, bias=None, out=None, tile_n: int = 0, pair: int = -1, split_k:
     if bias is not None:
         assert bias.dtype == torch.bfloat16 and bias.is_contiguous()
     from . import _count
+    if few_rows(M, N) and not packed and (tile_n, pair, split_k) == (0, -1, 0):
+        check(_lib.load().xllm_gemm_bf16_few(ptr(x2), w_ptr, ptr(o2), ptr(bias), M, N, K, x2.stride(0), w_ld, o2.stride(0),
+                                             stream()), "gemm_bf16_few")
+        _count()
+        return out.reshape(*x.shape[:-1], N)
     check(_lib.load().xllm_gemm_bf16(ptr(x2), w_ptr, ptr(o2), ptr(bias), M, N, K, x2.stride(0), w_ld,
                                      o2.stride(0), tile_n, pair, int(packed), split_k, stream()), "gemm_bf16")
     _count()
@@ -95,9 +118,11 @@ def gemm_act_mul(x, w_interleaved, act="silu", out=None):
     if out is None:
         out = torch.empty((T, N // 2), dtype=x.dtype, device=x.device)
     code, limit, alpha = glu.code(act)
-    check(_lib.load().xllm_gemm_bf16_act_mul(ptr(x), ptr(w_interleaved), ptr(out), T, N, K, x.stride(0),
-                                             w_interleaved.stride(0), out.stride(0), code + 1, limit, alpha, stream()),
-          "gemm_bf16_act_mul")
+    lib = _lib.load()
+    few = N % 128 == 0 and few_rows(T, N)
+    check((lib.xllm_gemm_bf16_act_mul_few if few else lib.xllm_gemm_bf16_act_mul)(
+        ptr(x), ptr(w_interleaved), ptr(out), T, N, K, x.stride(0), w_interleaved.stride(0), out.stride(0), code + 1, limit,
+        alpha, stream()), "gemm_bf16_act_mul")
     from . import _count
     _count()
     return out

@@ -17,6 +17,9 @@ from ._lib import F, I, L, P, check, ptr, stream
 _lib.register_signature("xllm_moe_route", [P, I, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P])
 _lib.register_signature("xllm_moe_route_ld", [P, L, I, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P])
 _lib.register_signature("xllm_moe_offsets", [P, P, P, P, I, I, I, P])
+_lib.register_signature("xllm_moe_offsets_tile", [P, P, P, P, I, I, I, I, P])
+_lib.register_signature("xllm_moe_permute_fp8", [P, P, P, P, P, P, P, P, I, I, I, I, P])
+_lib.register_signature("xllm_gemm_bf16_grouped_few", [P, P, P, P, I, I, I, I, I, L, L, I, F, F, P])
 _lib.register_signature("xllm_moe_permute", [P, P, P, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_moe_finalize", [P, P, L, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_moe_grouped_simt", [P, P, P, P, I, I, I, L, L, I, P])
@@ -64,6 +67,17 @@ def fused_moe_reference(x, logits, w_gate_up, w_down, top_k, scoring="softmax", 
     return out.to(x.dtype)
 
 
+MIN_TILE = 16
+
+
+def row_tile(T, top_k, n_experts):
+    """Rows of a tile of the grouped products, none of which two experts share.  With few rows per expert the products are
+    bound by the experts' weights, and small tiles (csrc/kernels/gemm_few.cu) leave out the rows that are not there; an
+    expert with more rows than a tile reads its weights again for the next, from L2.  So: the smallest tile that holds
+    about 2.5 times the average, 128 (gemm_tcgen05.cu) beyond."""
+    return next((t for t in (16, 32, 64) if T * top_k * 5 <= 2 * t * n_experts), 128)
+
+
 class MoeWorkspace:
     """Static-size buffers of one MoE layer shape (sized for max_tokens; reusable across layers)."""
 
@@ -74,6 +88,7 @@ class MoeWorkspace:
         self.counts = torch.zeros(n_experts, **i32)
         self.offsets = torch.zeros(n_experts, **i32)
         self.tile_expert = torch.full((self.max_tiles,), -1, **i32)
+        self.small_tile_expert = torch.full(((max_tokens * top_k + n_local * (MIN_TILE - 1)) // MIN_TILE + 1,), -1, **i32)
         self.meta = torch.zeros(4, **i32)
         self.topk_ids = torch.zeros(max_tokens * top_k, **i32)
         self.slot = torch.zeros(max_tokens * top_k, **i32)
@@ -141,40 +156,58 @@ def fused_moe(x, logits, w_gate_up, w_down, top_k, scoring="softmax", bias=None,
     check(lib.xllm_moe_route_ld(ptr(logits), logits.stride(0), int(lf), ptr(bias), ptr(ws.topk_ids), ptr(ws.topk_w), ptr(ws.counts),
                              ptr(ws.slot), T, E, top_k, n_group, topk_group,
                              (0 if scoring == "softmax" else 1) + (2 if group_score == "max" else 0), int(renorm), float(scale), expert_begin, expert_begin + E_local, s), "moe_route")
-    check(lib.xllm_moe_offsets(ptr(ws.counts), ptr(ws.offsets), ptr(ws.tile_expert), ptr(ws.meta), E, ws.max_tiles,
-                               expert_begin, s), "moe_offsets")
-    check(lib.xllm_moe_permute(ptr(ws.xp), ptr(ws.rows_of), ptr(x), ptr(ws.topk_ids), ptr(ws.slot), ptr(ws.offsets),
-                               T, top_k, H, dt, s), "moe_permute")
+    simt = w_scales is None and (dt == 1 or H % 8 or I2 % 64 or inter % 8 or Y % 64)
+    tile = 128 if simt or I2 % 128 or Y % 128 else row_tile(T, top_k, E)
+    # rows that T tokens can take: a workspace is made for more
+    rows = min(ws.rows, (T * top_k + min(E_local, T * top_k) * (tile - 1) + tile - 1) // tile * tile)
+    te = ws.tile_expert if tile == 128 else ws.small_tile_expert
+    check(lib.xllm_moe_offsets_tile(ptr(ws.counts), ptr(ws.offsets), ptr(te), ptr(ws.meta), E, min(te.shape[0], rows // tile),
+                                    expert_begin, tile, s), "moe_offsets")
+    launches = 6
     if w_scales is not None:
+        # quantised once per token, then permuted; the activation is quantised where it is computed
         from . import fp8
-        xq, xs = fp8.quant_group128(ws.xp)
-        fp8.block_scaled_mm_grouped(xq, xs, w_gate_up, w_scales[0], ws.tile_expert, ws.h)
-        act_and_mul(ws.h, act, out=ws.a)
-        aq, as_ = fp8.quant_group128(ws.a)
-        fp8.block_scaled_mm_grouped(aq, as_, w_down, w_scales[1], ws.tile_expert, ws.y)
-    elif dt == 1 or H % 8 or I2 % 64 or inter % 8 or Y % 64:
+        q, qs = fp8.quant_group128(x)
+        xq, xs = ws.xp.view(torch.uint8).view(-1)[:rows * H].view(fp8.FP8).view(rows, H), \
+            torch.empty(rows, H // 128, dtype=torch.float32, device=x.device)
+        check(lib.xllm_moe_permute_fp8(ptr(xq), ptr(xs), ptr(ws.rows_of), ptr(q), ptr(qs), ptr(ws.topk_ids), ptr(ws.slot),
+                                       ptr(ws.offsets), T, top_k, H, H // 128, s), "moe_permute_fp8")
+        fp8.block_scaled_mm_grouped(xq, xs, w_gate_up, w_scales[0], te, ws.h[:rows], tile)
+        aq, as_ = fp8.act_quant_group128(ws.h[:rows], act, te, tile)
+        fp8.block_scaled_mm_grouped(aq, as_, w_down, w_scales[1], te, ws.y[:rows], tile)
+        launches = 5
+    else:
+        check(lib.xllm_moe_permute(ptr(ws.xp), ptr(ws.rows_of), ptr(x), ptr(ws.topk_ids), ptr(ws.slot), ptr(ws.offsets),
+                                   T, top_k, H, dt, s), "moe_permute")
+    if simt:
         # fp32, or sizes the tensor-core kernel does not take
-        simt = lambda a, w, c: check(lib.xllm_moe_grouped_simt(ptr(a), ptr(w), ptr(c), ptr(ws.tile_expert), ws.rows, c.shape[1],
-                                                               a.shape[1], a.stride(0), c.stride(0), dt, s), "moe_gemm_simt")
+        product = lambda a, w, c: check(lib.xllm_moe_grouped_simt(ptr(a), ptr(w), ptr(c), ptr(te), rows, c.shape[1],
+                                                                  a.shape[1], a.stride(0), c.stride(0), dt, s), "moe_gemm_simt")
         if interleaved:
             raise ValueError("interleaved expert rows need the tensor-core product")
-        simt(ws.xp, w_gate_up, ws.h)
-        act_and_mul(ws.h, act, out=ws.a)
-        simt(ws.a, w_down, ws.y)
-    else:
+        product(ws.xp, w_gate_up, ws.h)
+        act_and_mul(ws.h[:rows], act, out=ws.a[:rows])
+        product(ws.a, w_down, ws.y)
+    elif w_scales is None:
+        def grouped(a, w, c, n, k, *glu_args):
+            if tile != 128:
+                check(lib.xllm_gemm_bf16_grouped_few(ptr(a), ptr(w), ptr(c), ptr(te), tile, rows, n, k, E_local, k, c.shape[1],
+                                                     *(glu_args or (0, 0.0, 0.0)), s), "moe_gemm_few")
+            elif glu_args:
+                check(lib.xllm_gemm_bf16_grouped_act_mul(ptr(a), ptr(w), ptr(c), ptr(te), rows, n, k, E_local, k, c.shape[1],
+                                                         *glu_args, s), "moe_gemm_act")
+            else:
+                check(lib.xllm_gemm_bf16_grouped(ptr(a), ptr(w), ptr(c), ptr(te), rows, n, k, E_local, k, c.shape[1], s), "moe_gemm")
         if interleaved:
             code, limit, alpha = glu.code(act)
-            check(lib.xllm_gemm_bf16_grouped_act_mul(ptr(ws.xp), ptr(w_gate_up), ptr(ws.a), ptr(ws.tile_expert), ws.rows,
-                                                     I2, H, E_local, H, inter, code + 1, limit, alpha, s), "moe_gemm1_act")
+            grouped(ws.xp, w_gate_up, ws.a, I2, H, code + 1, limit, alpha)
         else:
-            check(lib.xllm_gemm_bf16_grouped(ptr(ws.xp), ptr(w_gate_up), ptr(ws.h), ptr(ws.tile_expert), ws.rows, I2, H,
-                                             E_local, H, I2, s), "moe_gemm1")
-            act_and_mul(ws.h, act, out=ws.a)
-        check(lib.xllm_gemm_bf16_grouped(ptr(ws.a), ptr(w_down), ptr(ws.y), ptr(ws.tile_expert), ws.rows, Y, inter,
-                                         E_local, inter, Y, s), "moe_gemm2")
+            grouped(ws.xp, w_gate_up, ws.h, I2, H)
+            act_and_mul(ws.h[:rows], act, out=ws.a[:rows])
+        grouped(ws.a, w_down, ws.y, Y, inter)
     if out is None:
         out = torch.empty_like(x)
     check(lib.xllm_moe_finalize(ptr(out), ptr(ws.y), Y, ptr(ws.rows_of), ptr(ws.topk_w), ptr(shared_out), T, top_k, H, dt, s),
           "moe_finalize")
-    _count(6)
+    _count(launches)
     return out
