@@ -8,8 +8,8 @@
 //
 //   gdn_conv_kernel   convolution -> bf16 rows, 1 / |q| and 1 / |k|, decays and betas
 //   gdn_step_kernel   one token per sequence, from there to the finished row; the state crosses HBM once in each direction
-//   gdn_scan_kernel   prompts: all sequences and heads at once, token by token in fp32 with the state in registers; the last
-//                     inputs of a sequence -> its convolution tail
+//   gdn_prep_kernel,  prompts: all sequences and heads at once, sixteen tokens at a time on the tensor cores (below); the last
+//   gdn_chunk_kernel  inputs of a sequence -> its convolution tail
 //   gdn_norm_kernel   prompts: norm, weight and gate
 //
 // Measured against the same layer as tensor operations around gdn.cu (one B200, 32 heads of 128 x 128, four prompts of up to
@@ -18,7 +18,7 @@
 //
 // A sequence whose rows in the batch are its first tokens (kv_len == number of rows) starts from zeros whatever its slot
 // holds; slot < 0 marks padding rows, which come out as zeros.  Built without fast-math: errors of a decay multiply up.
-#include "recurrence.cuh"
+#include "attn_common.cuh"
 #include "short_conv.cuh"
 
 namespace xllm {
@@ -37,12 +37,13 @@ struct GdnParams {
   int ba_gs;                  // stride of the blocks of a key head's value heads
   const bf16 *conv_w;         // [C, taps], the last tap is the current token's
   const bf16 *dt_bias, *a_log, *norm_w;
-  bf16 *yq, *yk, *yv;         // [rows, G, dk], [rows, G, dk], [rows, H, dv]
+  bf16 *yq, *yk, *yv;         // [rows, G, dkp], [rows, G, dkp], [rows, H, dvp]; dkp: 64 or 128, zeros behind dk; dvp: dv in eights
   float *fq, *fk;             // [rows, G]: factors that make yq, yk unit vectors (yq: scaled)
-  float2* gb;                 // [rows, H]: exp(g), beta
+  float2* gb;                 // [rows, H]: exp(g) (decode rows) or g, and beta
+  uint8_t* blobs;             // prompts: see GdnBlob
   float* o;                   // [rows, H, dv] (prompts)
   bf16* out;                  // [rows, H dv]
-  int n_decode, n_seqs, rows, H, G, dk, dv, taps;
+  int n_decode, n_seqs, rows, H, G, dk, dv, dkp, dvp, taps;
   float q_scale, eps;
   __host__ __device__ int64_t channels() const { return (int64_t)2 * G * dk + (int64_t)H * dv; }
 };
@@ -65,7 +66,8 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(GdnParams p) {
         const int64_t at = row * p.ba_ld + (int64_t)(n / r) * p.ba_gs + n % r;
         const float x = __bfloat162float(p.a[at]) + __bfloat162float(p.dt_bias[n]);
         const float sp = x > 20.f ? x : log1pf(expf(x));
-        p.gb[(int64_t)row * p.H + n] = make_float2(expf(-expf(__bfloat162float(p.a_log[n])) * sp), sigmoid_exact(__bfloat162float(p.b[at])));
+        const float g = -expf(__bfloat162float(p.a_log[n])) * sp;
+        p.gb[(int64_t)row * p.H + n] = make_float2(row < p.n_decode ? expf(g) : g, sigmoid_exact(__bfloat162float(p.b[at])));
       }
     return;
   }
@@ -75,8 +77,9 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(GdnParams p) {
   const bool on = c < d;
   const int64_t ch = (part == 2 ? (int64_t)2 * p.G * p.dk : (int64_t)part * p.G * p.dk) + (int64_t)h * d + c, C = p.channels();
   const bf16* x = (part == 2 ? p.v + (int64_t)(h / r) * p.v_gs + (h % r) * d : (part == 0 ? p.q : p.k) + (int64_t)h * p.qk_hs) + c;
-  bf16* y = (part == 0 ? p.yq : (part == 1 ? p.yk : p.yv)) + (int64_t)h * d + c;
-  const int64_t y_ld = (int64_t)(part == 2 ? p.H : p.G) * d;
+  const int dp = part == 2 ? p.dvp : p.dkp;
+  bf16* y = (part == 0 ? p.yq : (part == 1 ? p.yk : p.yv)) + (int64_t)h * dp + c;
+  const int64_t y_ld = (int64_t)(part == 2 ? p.H : p.G) * dp;
   float v[RUN + 3][4], w[4][4];                                     // w[taps back][channel]
 #pragma unroll
   for (int i = 0; i < RUN + 3; ++i) {
@@ -143,21 +146,21 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(GdnParams p) {
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      s[j] = on ? __bfloat162float(__float2bfloat16(s[j] * sigmoid_exact(s[j]))) : 0.f;
+      s[j] = on ? __bfloat162float(__float2bfloat16(silu_as<bf16>(s[j]))) : 0.f;
       ss += s[j] * s[j];
     }
     if (part < 2) {
       ss = warp_sum(ss);
       if (lane == 0) (part == 0 ? p.fq : p.fk)[(int64_t)row * p.G + h] = (part == 0 ? p.q_scale : 1.f) / sqrtf(ss + kGdnUnitEps);
     }
-    if (on) store_f32<4>(y + row * y_ld, s);
+    if (c < dp) store_f32<4>(y + row * y_ld, s);                     // zeros behind d
   }
 }
 
 // silu(z) times the normed and weighted output, in the model's order of roundings
 __device__ __forceinline__ bf16 gdn_finish(float o, float inv, bf16 w, float z) {
   const bf16 n = __float2bfloat16(o * inv);
-  return __float2bfloat16(__bfloat162float(__float2bfloat16(__bfloat162float(w) * __bfloat162float(n))) * (z * sigmoid_exact(z)));
+  return __float2bfloat16(__bfloat162float(__float2bfloat16(__bfloat162float(w) * __bfloat162float(n))) * silu_as<bf16>(z));
 }
 
 // ------------------------------------------------------------------------------------------------ decode
@@ -189,10 +192,10 @@ __global__ void __launch_bounds__(256, 2) gdn_step_kernel(GdnParams p) {
   const int r = p.H / p.G;
   const int64_t qk = (int64_t)b * p.G + h / r, row = (int64_t)b * p.H + h;
   if (tid < dk) {
-    qs[tid] = __bfloat162float(p.yq[qk * dk + tid]) * p.fq[qk];
-    ks[tid] = __bfloat162float(p.yk[qk * dk + tid]) * p.fk[qk];
+    qs[tid] = __bfloat162float(p.yq[qk * p.dkp + tid]) * p.fq[qk];
+    ks[tid] = __bfloat162float(p.yk[qk * p.dkp + tid]) * p.fk[qk];
   }
-  if (tid >= 128 && tid - 128 < dv) vs[tid - 128] = __bfloat162float(p.yv[row * dv + tid - 128]);
+  if (tid >= 128 && tid - 128 < dv) vs[tid - 128] = __bfloat162float(p.yv[row * p.dvp + tid - 128]);
   const float2 gb = p.gb[row];
   const float z = tid < dv ? __bfloat162float(p.z[b * p.z_ld + (int64_t)(h / r) * p.z_gs + (h % r) * dv + tid]) : 0.f;
   const bf16 w_out = tid < dv ? p.norm_w[tid] : __float2bfloat16(0.f);
@@ -240,30 +243,160 @@ __global__ void __launch_bounds__(256, 2) gdn_step_kernel(GdnParams p) {
   if (tid < dv) orow[tid] = gdn_finish(mine, inv, w_out, z);
 }
 
-// ------------------------------------------------------------------------------------------------ prompts: recurrence
-// grid (slices of 32 columns, heads, sequences), four warps of eight columns (recurrence.cuh).  A token costs one pass over
-// the state for S^T k, one that adds k u^T and takes S^T q, and no barrier.  The decay is no pass of its own: the registers
-// hold S / c with c the product of the decays since it was last multiplied in, which happens before it falls below 2^-40.
-// The next tile's vectors are on their way while one is worked on and meet their factors on the way into shared memory.
-constexpr int kGdnWarps = 4, kGdnCols = kGdnWarps * kRecCols;
+// ------------------------------------------------------------------------------------------------ prompts, chunks of 16
+// With G_t the sum of a chunk's g through token t, S_0 the state before the chunk, y the convolution's q and k rows and f their
+// factors,
+//
+//   A_ts = e^(G_t - G_s) f_t f_s y_t . y_s  (s < t),   P_ts = e^(G_t - G_s) fq_t f_s yq_t . y_s  (s <= t),
+//   M = (I + diag(beta) A)^-1 diag(beta),    U = M (V - diag(f e^G) Y S_0),    O = diag(fq e^G) Yq S_0 + P U,
+//   S <- e^(G_end) S_0 + Y^T diag(f e^(G_end - G)) U.
+//
+// Every decay is at most 1.  y and v are bf16 as the convolution leaves them, so that their products on the tensor cores are
+// exact and accumulate in fp32; S, U, M and P are fp32 values as three bf16 terms (24 bits), of which products below 2^-24 of
+// the largest are left out.  gdn_prep_kernel makes M, P and the factors, all chunks side by side; gdn_chunk_kernel walks the
+// chunks of a sequence: a warp owns 16 state columns for all of dk as accumulators of S^T, which are the A operand of S^T Y^T
+// without leaving the registers, as U^T is of the products behind it.
+//
+// Token by token in fp32 (states in registers, no barriers) the walk took 600 us for four prompts of 1024, 549, 842 and 366
+// tokens, 32 heads of 128 x 128 (one B200), some 1100 cycles a token in a chain of product, exchange, product.
+constexpr int kGC = 16, kGWarps = 4, kGCols = 16 * kGWarps, kGStages = 3, kGVld = kGCols + 8;
 
-template <int J>
-__global__ void __launch_bounds__(32 * kGdnWarps, 4) gdn_scan_kernel(GdnParams p) {
-  constexpr int DK = 32 * J, TT = kRecTile, NT = 32 * kGdnWarps;
-  __shared__ __align__(16) float ksm[2][TT][DK], qsm[2][TT][DK], vsm[2][TT][kGdnCols];
-  __shared__ float2 gsm[2][TT];
-  const int h = blockIdx.y, b = p.n_decode + blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rgrp = lane & 7, c0 = blockIdx.x * kGdnCols, lc = warp * kRecCols + (lane >> 3) * 2, col = c0 + lc;
-  const int r = p.H / p.G, g = h / r, dk = p.dk, dv = p.dv;
+struct GdnBlob {                             // bytes of one (chunk, head)
+  static constexpr int mat = kGC * kGC * 2;  // [16][16] bf16
+  static constexpr int m = 0, p = 3 * mat;   // three terms behind one another
+  static constexpr int f = 6 * mat;          // [16] float4: f e^G, fq e^G, f e^(G_end - G), e^(G_end)
+  static constexpr int bytes = f + kGC * 16;
+};
+// chunk i of prompt b: unique because a sequence of n rows has at most n / 16 + 1 chunks
+__host__ __device__ __forceinline__ int64_t gdn_chunk_slot(int64_t row0, int b, int i) { return row0 / kGC + b + i; }
+
+__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const auto pack = [](bf162 v) { return *reinterpret_cast<const uint32_t*>(&v); };
+  const bf162 h = __floats2bfloat162_rn(x, y);
+  const float2 hf = __bfloat1622float2(h);
+  const bf162 m = __floats2bfloat162_rn(x - hf.x, y - hf.y);
+  const float2 mf = __bfloat1622float2(m);
+  hi = pack(h);
+  mid = pack(m);
+  lo = pack(__floats2bfloat162_rn(x - hf.x - mf.x, y - hf.y - mf.y));
+}
+__device__ __forceinline__ void put3(bf16* at, int stride, float x) {
+  const bf16 h = __float2bfloat16(x), m = __float2bfloat16(x - __bfloat162float(h));
+  at[0] = h;
+  at[stride] = m;
+  at[2 * stride] = __float2bfloat16(x - __bfloat162float(h) - __bfloat162float(m));
+}
+
+// grid (chunks of a sequence, key heads, prompts), 128 threads: warps 0 and 1 take Y Y^T and Yq Y^T, then a warp a value head
+template <int DK>
+__global__ void __launch_bounds__(128) gdn_prep_kernel(GdnParams p) {
+  constexpr int LD = DK + 8, PC = DK / 8;
+  __shared__ __align__(16) bf16 rows[2][kGC][LD];                    // k, q
+  __shared__ float dots[2][kGC][kGC + 1], am[4][kGC][kGC + 1], gs[4][kGC], bs[4][kGC], ff[2][kGC];
+  const int g = blockIdx.y, b = p.n_decode + blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_wait();
   pdl_launch_dependents();
-  const int row0 = p.cu_q[b], n = p.cu_q[b + 1] - row0, slot = p.slots[b];
-  if (n <= 0 || slot < 0) return;
-  const bool fresh = p.kv_lens[b] == n, mine = col < dv;
-  float* S = p.state + (((int64_t)slot * p.H + h) * dk) * dv + col;
-  StateColumns<J> st;
-  st.load(S, dk, dv, rgrp, mine && !fresh);
-  if (blockIdx.x == 0 && n > 1) {                                   // the convolution has read the tails
+  const int first = p.cu_q[b], n_seq = p.cu_q[b + 1] - first, i0 = blockIdx.x * kGC;
+  if (i0 >= n_seq || p.slots[b] < 0) return;
+  const int n = min(kGC, n_seq - i0), row0 = first + i0, r = p.H / p.G;
+  for (int i = tid; i < 2 * kGC * PC; i += 128) {
+    const int which = i / (kGC * PC), t = i / PC % kGC, c = (i % PC) * 8;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (t < n) v = *reinterpret_cast<const uint4*>((which ? p.yq : p.yk) + ((int64_t)(row0 + t) * p.G + g) * DK + c);
+    *reinterpret_cast<uint4*>(&rows[which][t][c]) = v;
+  }
+  if (tid < 2 * kGC) {
+    const int t = tid % kGC;
+    ff[tid / kGC][t] = t < n ? (tid < kGC ? p.fk : p.fq)[(int64_t)(row0 + t) * p.G + g] : 0.f;
+  }
+  __syncthreads();
+  const int ta = lane >> 2, kc = (lane & 3) * 2;
+  if (warp < 2) {
+    float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+    for (int k = 0; k < DK; k += 16) {
+      const auto at = [&](int which, int t, int c) { return *reinterpret_cast<const uint32_t*>(&rows[which][t][k + c]); };
+      const uint32_t a[4] = {at(warp, ta, kc), at(warp, ta + 8, kc), at(warp, ta, kc + 8), at(warp, ta + 8, kc + 8)};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) mma_bf16_16816(d[j], a, at(0, 8 * j + ta, kc), at(0, 8 * j + ta, kc + 8));
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dots[warp][ta + (e >> 1) * 8][8 * j + kc + (e & 1)] = d[j][e];
+  }
+  __syncthreads();
+  for (int i = warp; i < r; i += 4) {
+    const int h = g * r + i;
+    uint8_t* blob = p.blobs + (gdn_chunk_slot(first, blockIdx.z, blockIdx.x) * p.H + h) * GdnBlob::bytes;
+    float G = 0.f;
+    if (lane < kGC) {
+      const float2 gb = lane < n ? p.gb[(int64_t)(row0 + lane) * p.H + h] : make_float2(0.f, 0.f);
+      G = gb.x;                                                      // g: rows behind the last one add nothing
+      bs[warp][lane] = gb.y;                                         // and have beta 0
+    }
+#pragma unroll
+    for (int o = 1; o < kGC; o <<= 1) {
+      const float x = __shfl_up_sync(0xffffffffu, G, o);
+      if (lane >= o) G += x;
+    }
+    const float end = __shfl_sync(0xffffffffu, G, kGC - 1);
+    if (lane < kGC) {
+      gs[warp][lane] = G;
+      const float e = expf(G);
+      reinterpret_cast<float4*>(blob + GdnBlob::f)[lane] =
+          make_float4(ff[0][lane] * e, ff[1][lane] * e, ff[0][lane] * expf(end - G), expf(end));
+    }
+    __syncwarp();
+    for (int x = lane; x < kGC * kGC; x += 32) {
+      const int t = x >> 4, s = x & 15;
+      const float e = s <= t ? expf(gs[warp][t] - gs[warp][s]) * ff[0][s] : 0.f;
+      am[warp][t][s] = s < t ? bs[warp][t] * ff[0][t] * e * dots[0][t][s] : 0.f;
+      put3(reinterpret_cast<bf16*>(blob + GdnBlob::p) + x, kGC * kGC, ff[1][t] * e * dots[1][t][s]);
+    }
+    __syncwarp();
+    if (lane < kGC) {                                                // column `lane` of the inverse by forward substitution
+      float x[kGC];
+      const float bt = bs[warp][lane];
+#pragma unroll
+      for (int t = 0; t < kGC; ++t) {
+        float y = t == lane ? 1.f : 0.f;
+#pragma unroll
+        for (int s = 0; s < t; ++s) y -= am[warp][t][s] * x[s];
+        x[t] = y;
+        put3(reinterpret_cast<bf16*>(blob + GdnBlob::m) + t * kGC + lane, kGC * kGC, y * bt);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// grid (slices of 64 columns, heads, prompts)
+template <int DK>
+__global__ void __launch_bounds__(32 * kGWarps, 2) gdn_chunk_kernel(GdnParams p) {
+  constexpr int CH = DK / 8, NT = 32 * kGWarps, TILE = kGC * DK * 2;
+  constexpr int V_OFF = 2 * TILE, B_OFF = V_OFF + kGC * kGVld * 2, STAGE = (B_OFF + GdnBlob::bytes + 127) / 128 * 128;
+  static_assert(kGStages * STAGE <= 48 * 1024, "static limit of dynamic shared memory");
+  extern __shared__ __align__(128) uint8_t smem[];
+  const uint32_t sb = smem_u32(smem);
+  const int h = blockIdx.y, b = p.n_decode + blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r = p.H / p.G, g = h / r, dk = p.dk, dv = p.dv, dvp = p.dvp, c0 = blockIdx.x * kGCols;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int row0 = p.cu_q[b], n_all = p.cu_q[b + 1] - row0, slot = p.slots[b];
+  if (n_all <= 0 || slot < 0) return;
+  const bool fresh = p.kv_lens[b] == n_all, works = c0 + warp * 16 < dv;
+  float* S = p.state + (((int64_t)slot * p.H + h) * dk) * dv;
+  const int vloc = warp * 16 + (lane >> 2), vrow = c0 + vloc, kc = (lane & 3) * 2;
+  float acc[DK / 8][4];                      // S^T: rows (value columns) lane / 4, + 8; key channels 8 nt + kc, + 1
+#pragma unroll
+  for (int nt = 0; nt < DK / 8; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = nt * 8 + kc + (e & 1), v = vrow + (e >> 1) * 8;
+      acc[nt][e] = (!fresh && c < dk && v < dv) ? S[(int64_t)c * dv + v] : 0.f;
+    }
+  if (blockIdx.x == 0 && n_all > 1) {                               // the convolution has read the tails
     const int K1 = p.taps - 1;
     const int64_t C = p.channels();
     const bool qk = h % r == 0;
@@ -274,123 +407,156 @@ __global__ void __launch_bounds__(32 * kGdnWarps, 4) gdn_scan_kernel(GdnParams p
       bf16* tail = p.tail + ((int64_t)slot * C + ch) * K1;
       bf16 keep[3];
       for (int t = 0; t < K1; ++t) {                                // input t of the new tail, of tail | rows
-        const int at = n - K1 + t;
-        keep[t] = at >= 0 ? x[(row0 + at) * p.ld + c] : (fresh ? __float2bfloat16(0.f) : tail[n + t]);
+        const int at = n_all - K1 + t;
+        keep[t] = at >= 0 ? x[(row0 + at) * p.ld + c] : (fresh ? __float2bfloat16(0.f) : tail[n_all + t]);
       }
       for (int t = 0; t < K1; ++t) tail[t] = keep[t];
     }
   }
-  for (int i = tid; i < 2 * TT * DK; i += NT) (&ksm[0][0][0])[i] = (&qsm[0][0][0])[i] = 0.f;      // zeros behind dk
-  for (int i = tid; i < 2 * TT * kGdnCols; i += NT) (&vsm[0][0][0])[i] = 0.f;                     // and behind dv
-  __syncthreads();
-  // a thread's share of a tile: four values of q and k (FQ times), four of v, the decay and beta of one token
-  constexpr int FQ = TT * DK / 4 / NT;
-  uint2 qr[FQ], kr[FQ], vr;
-  float qf[FQ], kf_[FQ];
-  float2 gr = make_float2(1.f, 0.f);
-  const int vt = tid / (kGdnCols / 4), vc = (tid % (kGdnCols / 4)) * 4;
-  static_assert(TT * kGdnCols / 4 == NT, "one v load per thread");
-  const auto fetch = [&](int t0) {
-    const int m = min(TT, n - t0);
+  const int chunks = (n_all + kGC - 1) / kGC;
+  const uint8_t* blobs = p.blobs + (gdn_chunk_slot(row0, blockIdx.z, 0) * p.H + h) * GdnBlob::bytes;
+  const auto load = [&](int j) {
+    if (j < chunks) {
+      const uint32_t st = sb + (j % kGStages) * STAGE;
+      for (int i = tid; i < 2 * kGC * CH; i += NT) {
+        const int which = i / (kGC * CH), t = i / CH % kGC, c = i % CH;
+        const bool ok = j * kGC + t < n_all;
+        const int64_t row = row0 + (ok ? j * kGC + t : 0);
+        cp_async16(st + which * TILE + swz<CH>(t, c), (which ? p.yq : p.yk) + (row * p.G + g) * DK + c * 8, ok);
+      }
+      for (int i = tid; i < kGC * (kGCols / 8); i += NT) {
+        const int t = i / (kGCols / 8), c = (i % (kGCols / 8)) * 8;
+        const bool ok = j * kGC + t < n_all && c0 + c < dvp;
+        const int64_t row = row0 + (ok ? j * kGC + t : 0);
+        cp_async16(st + V_OFF + (t * kGVld + c) * 2, p.yv + (row * p.H + h) * dvp + (ok ? c0 + c : 0), ok);
+      }
+      const uint8_t* src = blobs + (int64_t)j * p.H * GdnBlob::bytes;
+      for (int i = tid; i < GdnBlob::bytes / 16; i += NT) cp_async16(st + B_OFF + i * 16, src + i * 16, true);
+    }
+    cp_async_commit();
+  };
 #pragma unroll
-    for (int i = 0; i < FQ; ++i) {
-      const int e = tid + i * NT, t = e / (DK / 4), c = (e % (DK / 4)) * 4;
-      if (t < m && c < dk) {
-        const int64_t at = (int64_t)(row0 + t0 + t) * p.G + g;
-        qr[i] = *reinterpret_cast<const uint2*>(p.yq + at * dk + c);
-        kr[i] = *reinterpret_cast<const uint2*>(p.yk + at * dk + c);
-        qf[i] = p.fq[at];
-        kf_[i] = p.fk[at];
+  for (int s = 0; s < kGStages - 1; ++s) load(s);
+  const int arow = (lane & 7) + (((lane >> 3) & 1) << 3), acb = lane >> 4;
+  const int brow = (lane & 7) + ((lane >> 4) << 3), bcb = (lane >> 3) & 1;
+  for (int j = 0; j < chunks; ++j) {
+    const int n = min(kGC, n_all - j * kGC);
+    cp_async_wait<kGStages - 2>();
+    __syncthreads();                         // chunk j is here, and everybody is done with the stage that is filled next
+    load(j + kGStages - 1);
+    if (!works) continue;
+    const uint32_t st = sb + (j % kGStages) * STAGE;
+    const uint8_t* stp = smem + (j % kGStages) * STAGE;
+    float w[2][4], wl[2][4], o[2][4], ol[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[i][e] = wl[i][e] = o[i][e] = ol[i][e] = 0.f;
+    // ---- S^T Y^T, S^T Yq^T
+#pragma unroll
+    for (int kk = 0; kk < DK / 16; ++kk) {
+      uint32_t kf[4], qf[4], hi[4], mid[4], lo[4];
+      const uint32_t at = st + swz<CH>(brow, kk * 2 + bcb);
+      ldmatrix_x4(kf[0], kf[1], kf[2], kf[3], at);
+      ldmatrix_x4(qf[0], qf[1], qf[2], qf[3], at + TILE);
+      split3(acc[2 * kk][0], acc[2 * kk][1], hi[0], mid[0], lo[0]);
+      split3(acc[2 * kk][2], acc[2 * kk][3], hi[1], mid[1], lo[1]);
+      split3(acc[2 * kk + 1][0], acc[2 * kk + 1][1], hi[2], mid[2], lo[2]);
+      split3(acc[2 * kk + 1][2], acc[2 * kk + 1][3], hi[3], mid[3], lo[3]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        mma_bf16_16816(w[i], hi, kf[2 * i], kf[2 * i + 1]);
+        mma_bf16_16816(o[i], hi, qf[2 * i], qf[2 * i + 1]);
+        mma_bf16_16816(wl[i], mid, kf[2 * i], kf[2 * i + 1]);
+        mma_bf16_16816(ol[i], mid, qf[2 * i], qf[2 * i + 1]);
+        mma_bf16_16816(wl[i], lo, kf[2 * i], kf[2 * i + 1]);
+        mma_bf16_16816(ol[i], lo, qf[2 * i], qf[2 * i + 1]);
       }
     }
-    if (vt < m && c0 + vc < dv) vr = *reinterpret_cast<const uint2*>(p.yv + ((int64_t)(row0 + t0 + vt) * p.H + h) * dv + c0 + vc);
-    if (tid < m) gr = p.gb[(int64_t)(row0 + t0 + tid) * p.H + h];
-  };
-  const auto widen = [](uint2 u, float f) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const bf162*>(&u.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const bf162*>(&u.y));
-    return make_float4(a.x * f, a.y * f, b.x * f, b.y * f);
-  };
-  const auto put = [&](int t0, int buf) {
-    const int m = min(TT, n - t0);
+    // ---- U^T = (V - W)^T M^T
+    const float4* fs = reinterpret_cast<const float4*>(stp + B_OFF + GdnBlob::f);
+    const bf16* vs = reinterpret_cast<const bf16*>(stp + V_OFF);
+    float4 f[2][2];                          // of tokens 8 i + kc, + 1
 #pragma unroll
-    for (int i = 0; i < FQ; ++i) {
-      const int e = tid + i * NT, t = e / (DK / 4), c = (e % (DK / 4)) * 4;
-      if (t < m && c < dk) {
-        *reinterpret_cast<float4*>(&qsm[buf][t][c]) = widen(qr[i], qf[i]);
-        *reinterpret_cast<float4*>(&ksm[buf][t][c]) = widen(kr[i], kf_[i]);
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) f[i][e] = fs[8 * i + kc + e];
+    uint32_t xh[4], xm[4], xl[4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const bf16* v = vs + (8 * i + kc) * kGVld + vloc + 8 * u;
+        split3(__bfloat162float(v[0]) - f[i][0].x * (w[i][2 * u] + wl[i][2 * u]),
+               __bfloat162float(v[kGVld]) - f[i][1].x * (w[i][2 * u + 1] + wl[i][2 * u + 1]), xh[2 * i + u], xm[2 * i + u], xl[2 * i + u]);
+      }
+    const uint32_t small = st + B_OFF + (uint32_t)(brow * kGC * 2 + bcb * 16);
+    float uu[2][4], pu[2][4];
+    // X^T times a matrix of three terms, the smallest products first
+    const auto product = [&](float (&d)[2][4], int at) {
+      uint32_t t0[4], t1[4], t2[4];
+      ldmatrix_x4(t0[0], t0[1], t0[2], t0[3], small + at);
+      ldmatrix_x4(t1[0], t1[1], t1[2], t1[3], small + at + GdnBlob::mat);
+      ldmatrix_x4(t2[0], t2[1], t2[2], t2[3], small + at + 2 * GdnBlob::mat);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[i][e] = 0.f;
+        mma_bf16_16816(d[i], xl, t0[2 * i], t0[2 * i + 1]);
+        mma_bf16_16816(d[i], xm, t1[2 * i], t1[2 * i + 1]);
+        mma_bf16_16816(d[i], xh, t2[2 * i], t2[2 * i + 1]);
+        mma_bf16_16816(d[i], xm, t0[2 * i], t0[2 * i + 1]);
+        mma_bf16_16816(d[i], xh, t1[2 * i], t1[2 * i + 1]);
+        mma_bf16_16816(d[i], xh, t0[2 * i], t0[2 * i + 1]);
+      }
+    };
+    product(uu, GdnBlob::m);
+    // ---- O^T
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) split3(uu[i][2 * u], uu[i][2 * u + 1], xh[2 * i + u], xm[2 * i + u], xl[2 * i + u]);
+    product(pu, GdnBlob::p);
+    // ---- S^T <- e^(G_end) S^T + U^T diag(f e^(G_end - G)) Y
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        split3(uu[i][2 * u] * f[i][0].z, uu[i][2 * u + 1] * f[i][1].z, xh[2 * i + u], xm[2 * i + u], xl[2 * i + u]);
+    const float end = f[0][0].w;
+#pragma unroll
+    for (int nt = 0; nt < DK / 8; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[nt][e] *= end;
+#pragma unroll
+    for (int kk = 0; kk < DK / 16; ++kk) {
+      uint32_t kf[4];
+      ldmatrix_x4_trans(kf[0], kf[1], kf[2], kf[3], st + swz<CH>(arow, kk * 2 + acb));
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        mma_bf16_16816(acc[2 * kk + i], xl, kf[2 * i], kf[2 * i + 1]);
+        mma_bf16_16816(acc[2 * kk + i], xm, kf[2 * i], kf[2 * i + 1]);
+        mma_bf16_16816(acc[2 * kk + i], xh, kf[2 * i], kf[2 * i + 1]);
       }
     }
-    if (vt < m && c0 + vc < dv) *reinterpret_cast<float4*>(&vsm[buf][vt][vc]) = widen(vr, 1.f);
-    if (tid < m) gsm[buf][tid] = gr;
-  };
-  fetch(0);
-  put(0, 0);
-  __syncthreads();
-  int buf = 0;
-  float c = 1.f;
-  for (int t0 = 0; t0 < n; t0 += TT, buf ^= 1) {
-    const bool more = t0 + TT < n;
-    if (more) fetch(t0 + TT);
-    const int m = min(TT, n - t0);
-    float* orow = p.o + ((int64_t)(row0 + t0) * p.H + h) * dv + col + (lane & 1);
-    const bool writes = rgrp < 2 && col + (lane & 1) < dv;
-#pragma unroll 2
-    for (int t = 0; t < m; ++t) {
-      const float2 gb = gsm[buf][t];
-      c *= gb.x;
-      if (c < 0x1p-40f) {                                           // uniform over the block
-        const f2 cc = pack_f2(c, c);
+    const int64_t row = row0 + j * kGC;
 #pragma unroll
-        for (int j = 0; j < 2 * J; ++j) {
-          st.s[0][j] = mul_f2(st.s[0][j], cc);
-          st.s[1][j] = mul_f2(st.s[1][j], cc);
-        }
-        c = 1.f;
-      }
-      const float bc = gb.y / c;
-      f2 kf[2 * J], qv[2 * J];
-      load_rows<J>(&ksm[buf][t][0], rgrp, kf);
-      f2 d0 = 0, d1 = 0, e0 = 0, e1 = 0;                            // packed zeros
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 2 * J; j += 2) {
-        d0 = fma_f2(st.s[0][j], kf[j], d0);
-        d1 = fma_f2(st.s[1][j], kf[j], d1);
-        e0 = fma_f2(st.s[0][j + 1], kf[j + 1], e0);
-        e1 = fma_f2(st.s[1][j + 1], kf[j + 1], e1);
+      for (int e = 0; e < 4; ++e) {
+        const int t = 8 * i + kc + (e & 1), v = vrow + (e >> 1) * 8;
+        if (t < n && v < dv) p.o[((row + t) * p.H + h) * dv + v] = f[i][e & 1].y * (o[i][e] + ol[i][e]) + pu[i][e];
       }
-      const float2 a0 = unpack_f2(add_f2(d0, e0)), a1 = unpack_f2(add_f2(d1, e1));
-      const float k0 = sum_row_groups(a0.x + a0.y), k1 = sum_row_groups(a1.x + a1.y);
-      const float2 v = *reinterpret_cast<const float2*>(&vsm[buf][t][lc]);
-      const float u0 = bc * (v.x - c * k0), u1 = bc * (v.y - c * k1);
-      const f2 w0 = pack_f2(u0, u0), w1 = pack_f2(u1, u1);
-      load_rows<J>(&qsm[buf][t][0], rgrp, qv);
-      d0 = d1 = e0 = e1 = 0;
-#pragma unroll
-      for (int j = 0; j < 2 * J; j += 2) {
-        st.s[0][j] = fma_f2(kf[j], w0, st.s[0][j]);
-        st.s[1][j] = fma_f2(kf[j], w1, st.s[1][j]);
-        st.s[0][j + 1] = fma_f2(kf[j + 1], w0, st.s[0][j + 1]);
-        st.s[1][j + 1] = fma_f2(kf[j + 1], w1, st.s[1][j + 1]);
-        d0 = fma_f2(st.s[0][j], qv[j], d0);
-        d1 = fma_f2(st.s[1][j], qv[j], d1);
-        e0 = fma_f2(st.s[0][j + 1], qv[j + 1], e0);
-        e1 = fma_f2(st.s[1][j + 1], qv[j + 1], e1);
-      }
-      const float2 y0 = unpack_f2(add_f2(d0, e0)), y1 = unpack_f2(add_f2(d1, e1));
-      const float y = c * sum_row_groups_2(y0.x + y0.y, y1.x + y1.y);
-      if (writes) orow[(int64_t)t * p.H * dv] = y;
-    }
-    if (more) put(t0 + TT, buf ^ 1);             // that buffer was last read before the barrier at the end of the last tile
-    __syncthreads();
   }
-  const f2 cc = pack_f2(c, c);
+  cp_async_wait<0>();
+  if (!works) return;
 #pragma unroll
-  for (int j = 0; j < 2 * J; ++j) {
-    st.s[0][j] = mul_f2(st.s[0][j], cc);
-    st.s[1][j] = mul_f2(st.s[1][j], cc);
-  }
-  if (mine) st.store(S, dk, dv, rgrp);
+  for (int nt = 0; nt < DK / 8; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = nt * 8 + kc + (e & 1), v = vrow + (e >> 1) * 8;
+      if (c < dk && v < dv) S[(int64_t)c * dv + v] = acc[nt][e];
+    }
 }
 
 // one warp per (row, head); a lane owns four neighbouring channels
@@ -449,21 +615,26 @@ XLLM_API int xllm_sigmoid_gate(void* out, const void* gate, int64_t ld, int hs, 
 }
 
 // Sequences 0 .. n_decode - 1 have one row each (rows 0 .. n_decode - 1), the others any number of rows behind them.
-// dk, dv <= 128 and multiples of 4, taps 2 .. 4, all rows and heads 8-byte aligned.  Scratch: yq, yk [rows, G, dk],
-// yv [rows, H, dv] bf16; fq, fk [rows, G], gb [rows, H, 2] fp32; o [rows, H, dv] fp32 where there are prompts.
+// dk, dv <= 128 and multiples of 4, taps 2 .. 4, all rows and heads 8-byte aligned; no prompt has more than max_q_len rows.
+// Scratch: yq, yk [rows, G, 64 or 128], yv [rows, H, dv in eights] bf16; fq, fk [rows, G], gb [rows, H, 2] fp32; where there
+// are prompts o [rows, H, dv] fp32 and xllm_gdn_blob_bytes() bytes.
+XLLM_API int64_t xllm_gdn_blob_bytes(int rows, int prompts, int H) {
+  return (xllm::gdn_chunk_slot(rows, prompts, 1) + 1) * H * xllm::GdnBlob::bytes;
+}
 XLLM_API int xllm_gdn_layer(void* state, void* tail, const void* slots, const void* cu_q, const void* kv_lens, const void* q,
                             const void* k, const void* v, const void* z, int64_t ld, int64_t z_ld, int qk_hs, int v_gs, int z_gs,
                             const void* b, const void* a, int64_t ba_ld, int ba_gs, const void* conv_w, const void* dt_bias,
                             const void* a_log, const void* norm_w, void* yq, void* yk, void* yv, void* fq, void* fk, void* gb,
-                            void* o, void* out, int n_decode, int n_seqs, int rows, int H, int G, int dk, int dv, int taps,
-                            float q_scale, float eps, void* stream) {
+                            void* o, void* blobs, void* out, int n_decode, int n_seqs, int rows, int max_q_len, int H, int G,
+                            int dk, int dv, int taps, float q_scale, float eps, void* stream) {
   using namespace xllm;
   if (rows <= 0 || n_seqs <= 0) return 0;
   const auto al8 = [](const void* x) { return (((uintptr_t)x) & 7) == 0; };
   if (H <= 0 || G <= 0 || H % G != 0 || dk <= 0 || dk > 128 || dk % 4 != 0 || dv <= 0 || dv > 128 || dv % 4 != 0 || taps < 2 ||
       taps > 4 || n_decode > rows || n_decode > n_seqs || ld % 4 != 0 || z_ld % 4 != 0 || qk_hs % 4 != 0 || v_gs % 4 != 0 ||
       z_gs % 4 != 0 || !al8(q) || !al8(k) || !al8(v) || !al8(z) || !al8(out) || !al8(yq) || !al8(yk) || !al8(yv) || !al8(tail) || !al8(conv_w) ||
-      (((uintptr_t)state) & 15) != 0)
+      ((((uintptr_t)state | (uintptr_t)yq | (uintptr_t)yk | (uintptr_t)yv | (uintptr_t)blobs) & 15) != 0) ||
+      (n_seqs > n_decode && (o == nullptr || blobs == nullptr || max_q_len <= 0)))
     return (int)cudaErrorInvalidValue;
   GdnParams p;
   p.state = (float*)state; p.tail = (bf16*)tail; p.slots = (const int32_t*)slots; p.cu_q = (const int32_t*)cu_q;
@@ -471,24 +642,31 @@ XLLM_API int xllm_gdn_layer(void* state, void* tail, const void* slots, const vo
   p.ld = ld; p.z_ld = z_ld; p.qk_hs = qk_hs; p.v_gs = v_gs; p.z_gs = z_gs; p.b = (const bf16*)b; p.a = (const bf16*)a;
   p.ba_ld = ba_ld; p.ba_gs = ba_gs; p.conv_w = (const bf16*)conv_w; p.dt_bias = (const bf16*)dt_bias;
   p.a_log = (const bf16*)a_log; p.norm_w = (const bf16*)norm_w; p.yq = (bf16*)yq; p.yk = (bf16*)yk; p.yv = (bf16*)yv;
-  p.fq = (float*)fq; p.fk = (float*)fk; p.gb = (float2*)gb; p.o = (float*)o; p.out = (bf16*)out;
+  p.fq = (float*)fq; p.fk = (float*)fk; p.gb = (float2*)gb; p.o = (float*)o; p.blobs = (uint8_t*)blobs;
+  p.out = (bf16*)out; p.dkp = dk <= 64 ? 64 : 128; p.dvp = (dv + 7) & ~7;
   p.n_decode = n_decode; p.n_seqs = n_seqs; p.rows = rows; p.H = H; p.G = G; p.dk = dk; p.dv = dv; p.taps = taps;
   p.q_scale = q_scale; p.eps = eps;
   cudaStream_t s = (cudaStream_t)stream;
-  // runs of four rows read an input once instead of four times; few rows need the warps more than the reuse
-  const int items = 2 * G + H + 1, run = rows > 128 ? 4 : 1;
+  // runs of eight rows read eleven inputs of a channel where eight single rows read 32; few rows need the warps more than
+  // the reuse
+  const int items = 2 * G + H + 1, run = rows > 128 ? 8 : 1;
   const dim3 grid((unsigned)((((int64_t)rows + run - 1) / run * items + 7) / 8));
   const auto conv = [&](auto kernel) { launch_pdl(kernel, grid, dim3(256), 0, s, p); };
-  if (taps == 4) conv(run == 4 ? gdn_conv_kernel<4, 3> : gdn_conv_kernel<1, 3>);
-  else if (taps == 3) conv(run == 4 ? gdn_conv_kernel<4, 2> : gdn_conv_kernel<1, 2>);
-  else conv(run == 4 ? gdn_conv_kernel<4, 1> : gdn_conv_kernel<1, 1>);
+  if (taps == 4) conv(run > 1 ? gdn_conv_kernel<8, 3> : gdn_conv_kernel<1, 3>);
+  else if (taps == 3) conv(run > 1 ? gdn_conv_kernel<8, 2> : gdn_conv_kernel<1, 2>);
+  else conv(run > 1 ? gdn_conv_kernel<8, 1> : gdn_conv_kernel<1, 1>);
   int rc = XLLM_LAUNCH_CHECK();
   if (rc != 0) return rc;
   if (n_seqs > n_decode) {
-    const dim3 sg((dv + kGdnCols - 1) / kGdnCols, H, n_seqs - n_decode), sb(32 * kGdnWarps);
-    if (dk <= 32) launch_pdl(gdn_scan_kernel<1>, sg, sb, 0, s, p);
-    else if (dk <= 64) launch_pdl(gdn_scan_kernel<2>, sg, sb, 0, s, p);
-    else launch_pdl(gdn_scan_kernel<4>, sg, sb, 0, s, p);
+    const int np = n_seqs - n_decode;
+    const dim3 pg((max_q_len + kGC - 1) / kGC, G, np), wg((dv + kGCols - 1) / kGCols, H, np);
+    const auto walk = [&](auto prep, auto chunk, int DK) {
+      const size_t smem = (size_t)kGStages * ((2 * kGC * DK * 2 + kGC * kGVld * 2 + GdnBlob::bytes + 127) / 128 * 128);
+      launch_pdl(prep, pg, dim3(128), 0, s, p);
+      launch_pdl(chunk, wg, dim3(32 * kGWarps), smem, s, p);
+    };
+    if (p.dkp == 64) walk(gdn_prep_kernel<64>, gdn_chunk_kernel<64>, 64);
+    else walk(gdn_prep_kernel<128>, gdn_chunk_kernel<128>, 128);
     if ((rc = XLLM_LAUNCH_CHECK()) != 0) return rc;
   }
   if (n_decode > 0) {

@@ -88,7 +88,7 @@ class GatedDeltaNet(Module):
             width = 2 * dk + 2 * r * dv
             strides = (width, width, width, 2 * r)
         out = self.fused(state.rec[self.lin_idx], state.conv[self.lin_idx], meta.state_slots, meta.cu_q, meta.kv_lens,
-                         meta.n_decode, y, k, v, z, b, a, *strides)
+                         meta.n_decode, y, k, v, z, b, a, *strides, max_q_len=meta.max_q_len)
         return self.out_proj(out)
 
     def forward(self, x, meta, state: LinearStateCache):

@@ -14,7 +14,8 @@ from ._lib import F, I, L, P, check, ptr, stream
 
 _lib.register_signature("xllm_gdn_decode_step", [P, P, P, P, P, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_gdn_prefill", [P, L, I, P, P, P, P, P, P, I, I, I, I, P])
-_lib.register_signature("xllm_gdn_layer", [P] * 9 + [L, L, I, I, I, P, P, L, I] + [P] * 12 + [I] * 8 + [F, F, P])
+_lib.register_signature("xllm_gdn_layer", [P] * 9 + [L, L, I, I, I, P, P, L, I] + [P] * 13 + [I] * 9 + [F, F, P])
+_lib.register_signature("xllm_gdn_blob_bytes", [I, I, I], L)
 _lib.register_signature("xllm_sigmoid_gate", [P, P, L, I, L, I, I, P])
 
 
@@ -38,9 +39,10 @@ class GatedDelta:
     a_log: torch.Tensor          # [nv]
     norm_w: torch.Tensor         # [dv]
 
-    def __call__(self, rec, tail, slots, cu_q, kv_lens, n_decode, q, k, v, z, b, a, qk_stride, v_stride, z_stride, ba_stride):
+    def __call__(self, rec, tail, slots, cu_q, kv_lens, n_decode, q, k, v, z, b, a, qk_stride, v_stride, z_stride, ba_stride,
+                 max_q_len=None):
         """rec [slots, nv, dk, dv] fp32 and tail [slots, channels, taps - 1] are advanced over the rows of the sequences
-        (the first `n_decode` have one each); returns the rows of the output projection [T, nv dv].  q, k, v, z, b, a: views
+        (the first `n_decode` have one each, none more than max_q_len, default: all); returns the rows of the output projection [T, nv dv].  q, k, v, z, b, a: views
         that start at head 0's place in the projection rows, rows by stride(0); `qk_stride`: between heads of q and k;
         `v_stride`, `z_stride`, `ba_stride`: between the blocks of the nv / nk value heads that share a key head."""
         T, dev, bf, f32 = q.shape[0], q.device, torch.bfloat16, torch.float32
@@ -54,18 +56,22 @@ class GatedDelta:
         assert rec.dtype == f32 and rec.is_contiguous() and rec.shape[1:] == (nv, dk, dv)
         assert tail.is_contiguous() and tail.shape[1:] == (2 * nk * dk + nv * dv, self.taps - 1)
         assert self.conv_w.is_contiguous()
-        yq, yk = torch.empty(T, nk, dk, dtype=bf, device=dev), torch.empty(T, nk, dk, dtype=bf, device=dev)
-        yv, out = torch.empty(T, nv, dv, dtype=bf, device=dev), torch.empty(T, nv * dv, dtype=bf, device=dev)
+        dkp, dvp = 64 if dk <= 64 else 128, (dv + 7) // 8 * 8
+        yq, yk = torch.empty(T, nk, dkp, dtype=bf, device=dev), torch.empty(T, nk, dkp, dtype=bf, device=dev)
+        yv, out = torch.empty(T, nv, dvp, dtype=bf, device=dev), torch.empty(T, nv * dv, dtype=bf, device=dev)
         factors = torch.empty(2 * T * (nk + nv), dtype=f32, device=dev)            # decays and betas first: pairs
         fq, fk = factors[2 * T * nv:], factors[T * (2 * nv + nk):]
-        o = torch.empty(T, nv, dv, dtype=f32, device=dev) if n > n_decode else None
+        o = blobs = None
+        if n > n_decode:
+            o = torch.empty(T, nv, dv, dtype=f32, device=dev)
+            blobs = torch.empty(_lib.load().xllm_gdn_blob_bytes(T, n - n_decode, nv), dtype=torch.uint8, device=dev)
         check(_lib.load().xllm_gdn_layer(
             ptr(rec), ptr(tail), ptr(slots), ptr(cu_q), ptr(kv_lens), ptr(q), ptr(k), ptr(v), ptr(z), q.stride(0), z.stride(0),
             qk_stride, v_stride, z_stride, ptr(b), ptr(a), a.stride(0), ba_stride, ptr(self.conv_w), ptr(self.dt_bias),
-            ptr(self.a_log), ptr(self.norm_w), ptr(yq), ptr(yk), ptr(yv), ptr(fq), ptr(fk), ptr(factors), ptr(o), ptr(out),
-            n_decode, n, T, nv, nk, dk, dv, self.taps, dk ** -0.5, self.eps, stream()), "gdn_layer")
+            ptr(self.a_log), ptr(self.norm_w), ptr(yq), ptr(yk), ptr(yv), ptr(fq), ptr(fk), ptr(factors), ptr(o), ptr(blobs), ptr(out),
+            n_decode, n, T, min(T, max_q_len or T), nv, nk, dk, dv, self.taps, dk ** -0.5, self.eps, stream()), "gdn_layer")
         from . import _count
-        _count(1 + int(n_decode > 0) + 2 * int(n > n_decode))
+        _count(1 + int(n_decode > 0) + 3 * int(n > n_decode))
         return out
 
 
