@@ -51,14 +51,22 @@ def test_fp8(M, N, K):
     _close(fp8.block_scaled_mm(a, a_s, w, w_s), want, 2 ** -8)
 
 
-@pytest.mark.parametrize("tile", [16, 32, 64])
+# more rows: single CTAs and pairs; rows, columns and K blocks that fill no tile, and more tiles than pairs
+@pytest.mark.parametrize("M,N,K", [(130, 2048, 256), (300, 7168, 640), (922, 7168, 2048), (1000, 8200, 384), (2100, 4352, 256)])
+def test_fp8_pairs(M, N, K):
+    test_fp8(M, N, K)
+
+
+@pytest.mark.parametrize("tile", [16, 32, 64, 256])
 @pytest.mark.parametrize("kind", ["bf16", "gated", "fp8"])
 def test_grouped(tile, kind):
     from xllm_b200.ops import _lib
     from xllm_b200.ops._lib import check, ptr, stream
     g = torch.Generator(device=DEV).manual_seed(tile)
     experts = torch.tensor([2, 0, -1, 2, 1, -1], dtype=torch.int32, device=DEV)
-    E, N, K, M = 3, 384, 640, 6 * tile
+    if tile == 256 and kind == "fp8":
+        pytest.skip("fp8 experts take tiles of up to 128 rows")
+    E, N, K, M = 3, 512 if tile == 256 else 384, 640, 6 * tile
     x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
     w = (torch.randn(E, N, K, device=DEV, generator=g) * K ** -0.5).bfloat16()
     out = torch.full((M, N // 2 if kind == "gated" else N), 7.0, device=DEV, dtype=torch.bfloat16)
@@ -69,6 +77,9 @@ def test_grouped(tile, kind):
         fp8.block_scaled_mm_grouped(a, a_s, wq, w_s, experts, out, tile)
         x = a.double() * a_s.double().repeat_interleave(128, 1)
         w = torch.stack([fp8.dequant_block128_ref(q, s, torch.float64) for q, s in parts])
+    elif tile == 256:
+        check(_lib.load().xllm_gemm_bf16_grouped_pair(ptr(x), ptr(w), ptr(out), ptr(experts), M, N, K, E, K, out.shape[1],
+                                                      int(kind == "gated"), 0.0, 0.0, stream()), "pair")
     else:
         check(_lib.load().xllm_gemm_bf16_grouped_few(ptr(x), ptr(w), ptr(out), ptr(experts), tile, M, N, K, E, K, out.shape[1],
                                                      int(kind == "gated"), 0.0, 0.0, stream()), "few")
@@ -94,8 +105,8 @@ def test_activation_and_its_quantisation(rows, d, act):
     assert torch.equal(got_s, want_s) and torch.equal(got_q.view(torch.uint8), want_q.view(torch.uint8))
 
 
-# (tokens, experts, chosen): one row tile after another, up to experts with more rows than a tile and to tiles of 128
-@pytest.mark.parametrize("T,E,K", [(1, 8, 2), (9, 32, 4), (40, 16, 4), (64, 8, 2), (130, 8, 2)])
+# (tokens, experts, chosen): one row tile after another up to pairs of CTAs, experts with more rows than a tile and with none
+@pytest.mark.parametrize("T,E,K", [(1, 8, 2), (9, 32, 4), (40, 16, 4), (64, 8, 2), (130, 8, 2), (447, 8, 2), (448, 8, 2), (1500, 8, 2)])
 @pytest.mark.parametrize("fp8_weights", [False, True])
 def test_expert_layer(T, E, K, fp8_weights):
     g = torch.Generator(device=DEV).manual_seed(T * E)
@@ -103,6 +114,7 @@ def test_expert_layer(T, E, K, fp8_weights):
     x = torch.randn(T, H, device=DEV, generator=g).bfloat16()
     logits = torch.randn(T, E, device=DEV, generator=g)
     logits[:, 1] += 3.0                                                          # a favourite
+    logits[:, 2] -= 30.0                                                         # and one that nobody wants
     up, down = ((torch.randn(E, *s, device=DEV, generator=g) * s[1] ** -0.5).bfloat16() for s in ((2 * I, H), (H, I)))
     scales = None
     if fp8_weights:

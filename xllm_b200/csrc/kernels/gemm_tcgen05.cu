@@ -526,6 +526,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (M + kBM - 1) / kBM, n_tiles = (N + BN - 1) / BN;
   const int total_tiles = m_tiles * n_tiles;
+  // Row tiles are neighbours, so that CTAs at work together share a tile's weights; grouped by expert, the column tiles of a row
+  // tile are: the experts' weights are read once either way, but all experts' rows (prompts: more than the L2 holds beside
+  // them) would be read again for every column tile (25 thousand rows of 2048 for 128 experts, one B200: 230 us, now 181 us
+  // with 1536 columns, 180 us, now 125 us for the product back).
+  const auto tile_m = [&](int t) { return tile_expert != nullptr ? t / n_tiles : t % m_tiles; };
+  const auto tile_n = [&](int t) { return tile_expert != nullptr ? t % n_tiles : t / m_tiles; };
   const int k_elems = mode.fp8 ? 2 * kBK : kBK;  // elements per 128-byte K block
   const int k_blocks = (K + k_elems - 1) / k_elems;
   const int ks = mode.ks;
@@ -567,12 +573,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
         const int tile = unit % total_tiles, kslice = unit / total_tiles;
         const int kb0 = kslice * kbs, kb1 = min(k_steps, kb0 + kbs);
-        const int m0 = (tile % m_tiles) * kBM;
-        int n0 = (tile / m_tiles) * BN;
+        const int m0 = tile_m(tile) * kBM;
+        int n0 = tile_n(tile) * BN;
         if (tile_expert != nullptr) {
           // grouped (MoE) mode: the row tile belongs to one expert, whose weights start
           // expert_rows * e rows into W; unused tail tiles are skipped by every role alike
-          const int e = tile_expert[tile % m_tiles];
+          const int e = tile_expert[tile_m(tile)];
           if (e < 0) continue;
           n0 += e * expert_rows;
         }
@@ -627,7 +633,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
       for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
         const int tile = unit % total_tiles, kslice = unit / total_tiles;
         const int kb0 = kslice * kbs, kb1 = min(k_steps, kb0 + kbs);
-        if (tile_expert != nullptr && tile_expert[tile % m_tiles] < 0) continue;
+        if (tile_expert != nullptr && tile_expert[tile_m(tile)] < 0) continue;
         const int acc = t & 1;
         const uint32_t use = (uint32_t)(t >> 1);
         ++t;
@@ -673,8 +679,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
     int steps_done = 0;  // ring steps of the units before this one: its parity says who owns the first stage
     for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
       const int tile = unit % total_tiles, kslice = unit / total_tiles;
-      if (tile_expert != nullptr && tile_expert[tile % m_tiles] < 0) continue;
-      const int m0 = (tile % m_tiles) * kBM, n0 = (tile / m_tiles) * BN;
+      if (tile_expert != nullptr && tile_expert[tile_m(tile)] < 0) continue;
+      const int m0 = tile_m(tile) * kBM, n0 = tile_n(tile) * BN;
       const int n_steps = min(k_steps, kslice * kbs + kbs) - kslice * kbs;
       const int acc = t & 1;
       const uint32_t use = (uint32_t)(t >> 1);
@@ -821,7 +827,7 @@ template <int BN, int STAGES, int KS, bool DUAL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DUAL ? 224 : 192, 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                               const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_ws,
-                              const bf16* __restrict__ bias, int M, int N, int K, int w_packed, const GemmMode mode, int* __restrict__ err_word) {
+                              const bf16* __restrict__ bias, int M, int N, int K, int w_packed, const int32_t* __restrict__ tile_expert, const GemmMode mode, int* __restrict__ err_word) {
   using S = GemmSmem2<BN, STAGES, KS>;
   constexpr int NACC = DUAL ? 2 : 1;  // accumulators per tile: one per MMA-issuing warp of the leader
   static_assert(2 * NACC * BN <= 512 && BN % 64 == 0, "TMEM has 512 columns; the epilogue works in 64-column chunks");
@@ -844,6 +850,10 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const _
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int m_tiles = (M + 2 * kBM - 1) / (2 * kBM), n_tiles = (N + BN - 1) / BN;
   const int total_tiles = m_tiles * n_tiles;
+  // grouped by expert (see gemm_bf16_tcgen05_kernel): a row tile of 256 belongs to one, expert e's weights are rows e N ..
+  const auto tile_m = [&](int t) { return tile_expert != nullptr ? t / n_tiles : t % m_tiles; };
+  const auto tile_n = [&](int t) { return tile_expert != nullptr ? t % n_tiles : t / m_tiles; };
+  const auto expert_of = [&](int t) { return tile_expert != nullptr ? tile_expert[tile_m(t)] : 0; };
   const int k_blocks = (K + kBK - 1) / kBK;
   const int ks = mode.ks;
   const int k_steps = (k_blocks + KS - 1) / KS;
@@ -884,8 +894,10 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const _
       for (int unit = pair; unit < total_units && ok; unit += n_pairs) {
         const int tile = unit % total_tiles, kslice = unit / total_tiles;
         const int kb0 = kslice * kbs, kb1 = min(k_steps, kb0 + kbs);
-        const int m0 = (tile % m_tiles) * (2 * kBM) + (int)rank * kBM;
-        const int n0 = (tile / m_tiles) * BN + (int)rank * (BN / 2);
+        const int e = expert_of(tile);
+        if (e < 0) continue;
+        const int m0 = tile_m(tile) * (2 * kBM) + (int)rank * kBM;
+        const int n0 = e * N + tile_n(tile) * BN + (int)rank * (BN / 2);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_cluster_warp(empty_bar(stage), phase ^ 1, abort_flag)) { ok = false; break; }
           const uint32_t a_dst = sbase + stage * S::STAGE_BYTES;
@@ -926,8 +938,9 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const _
       uint32_t phase = 0;
       bool ok = true;
       int t = 0;
-      for (int unit = pair; unit < total_units && ok; unit += n_pairs, ++t) {
+      for (int unit = pair; unit < total_units && ok; unit += n_pairs) {
         const int kslice = unit / total_tiles;
+        if (expert_of(unit % total_tiles) < 0) continue;
         const int kb0 = kslice * kbs, kb1 = min(k_steps, kb0 + kbs);
         const int acc = t & 1;
         const uint32_t use = (uint32_t)(t >> 1);
@@ -960,6 +973,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const _
         }
         if (ok && elect_one()) umma_commit_pair(tfull_bar(acc));
         __syncwarp();
+        ++t;
       }
     }
   } else {
@@ -969,12 +983,14 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const _
     bool ok = true;
     int t = 0, ebuf = 0;
     int steps_done = 0;
-    for (int unit = pair; unit < total_units && ok; unit += n_pairs, ++t) {
+    for (int unit = pair; unit < total_units && ok; unit += n_pairs) {
       const int tile = unit % total_tiles, kslice = unit / total_tiles;
-      const int m0 = (tile % m_tiles) * (2 * kBM) + (int)rank * kBM, n0 = (tile / m_tiles) * BN;
+      if (expert_of(tile) < 0) continue;
+      const int m0 = tile_m(tile) * (2 * kBM) + (int)rank * kBM, n0 = tile_n(tile) * BN;
       const int n_steps = min(k_steps, kslice * kbs + kbs) - kslice * kbs;
       const int acc = t & 1;
       const uint32_t use = (uint32_t)(t >> 1);
+      ++t;
       if (!mbar_wait_cluster(tfull_bar(acc), use & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t taddr = tmem_base + acc * NACC * BN + ((uint32_t)(q * 32) << 16);
@@ -1156,7 +1172,8 @@ static int launch_gemm(const void* a, const void* w, void* c, const void* bias, 
 template <int BN, int STAGES, int KS = 1, bool DUAL = false>
 static int launch_gemm_pair(const void* a, const void* w, void* c, const void* bias, int M, int N, int K, int64_t lda,
                             int64_t ldw, int64_t ldc, int max_ctas, int w_packed, cudaStream_t s, int split_k = 1,
-                            int act_mul = 0, float act_limit = 0.f, float act_alpha = 0.f) {
+                            int act_mul = 0, float act_limit = 0.f, float act_alpha = 0.f,
+                            const int32_t* tile_expert = nullptr, int n_experts = 1) {
   using S = GemmSmem2<BN, STAGES, KS>;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1173,7 +1190,7 @@ static int launch_gemm_pair(const void* a, const void* w, void* c, const void* b
   }
   CUtensorMap ta, tb, tc;
   const bool okb = w_packed ? make_tmap(&tb, w, (int64_t)N * (K / 64), 64, 64, BN / 2 < 64 ? BN / 2 : 64)
-                            : make_tmap(&tb, w, N, K, ldw, BN / 2);
+                            : make_tmap(&tb, w, (int64_t)N * n_experts, K, ldw, BN / 2);
   if (!make_tmap(&ta, a, M, K, lda, kBM) || !okb || !make_tmap(&tc, c, M, act_mul ? N / 2 : N, ldc, 32, false))
     return (int)cudaErrorInvalidValue;
   const int tiles = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + BN - 1) / BN);
@@ -1192,7 +1209,7 @@ static int launch_gemm_pair(const void* a, const void* w, void* c, const void* b
   const int units = tiles * mode.ks;
   int pairs = units < max_ctas / 2 ? units : max_ctas / 2;
   launch_pdl(gemm_bf16_tcgen05_pair_kernel<BN, STAGES, KS, DUAL>, dim3(2 * pairs), dim3(DUAL ? 224 : 192), S::TOTAL, s, ta, tb, tc, tws, (const bf16*)bias, M, N, K,
-                                                                            w_packed, mode, g_err_word[dev & 63]);
+                                                                            w_packed, tile_expert, mode, g_err_word[dev & 63]);
   return XLLM_LAUNCH_CHECK();
 }
 
@@ -1226,6 +1243,9 @@ XLLM_API int xllm_gemm_bf16_act_mul(const void* a, const void* w, void* c, int M
 // (tcgen05.ld), multiply by the block's scales and add into fp32 registers (eight warps: one output row
 // and 64 of the 128 columns per thread) while the MMA warp already fills the other buffer.  One tile is 128 x 128, so
 // the weight scale is one number per (tile, K block) and the activation scale one per (row, K block).
+// Bound by reading TMEM back, 64 KB per K block and tile: 922 x 36864 x 7168 reads 8.5 GB in 469 us (one B200), 18 TB/s, with the
+// tensor pipe 28 % active.  Pairs of CTAs on 256 x 256 (616 us), sixteen such warps (484 us) and scales fetched four blocks
+// ahead (486 us) read the same bytes and were not quicker.
 // Grouped form (MoE experts): `tile_expert[row tile]` names the expert of each 128-row tile (-1:
 // skip); expert e's weights start e * expert_rows rows into W and its scale rows e * expert_rows / 128
 // rows into w_scale.
@@ -1260,6 +1280,8 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (M + kBM - 1) / kBM, n_tiles = (N + BN - 1) / BN;
   const int total_tiles = m_tiles * n_tiles;
+  const auto tile_m = [&](int t) { return tile_expert != nullptr ? t / n_tiles : t % m_tiles; };   // as in gemm_bf16_tcgen05_kernel
+  const auto tile_n = [&](int t) { return tile_expert != nullptr ? t % n_tiles : t / m_tiles; };
   const int k_blocks = K / 128;
 
   if (threadIdx.x == 0) {
@@ -1293,10 +1315,10 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     bool ok = true;
     int armed = 0;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-      const int m0 = (tile % m_tiles) * kBM;
-      int n0 = (tile / m_tiles) * BN;
+      const int m0 = tile_m(tile) * kBM;
+      int n0 = tile_n(tile) * BN;
       if (tile_expert != nullptr) {
-        const int e = tile_expert[tile % m_tiles];
+        const int e = tile_expert[tile_m(tile)];
         if (e < 0) continue;
         n0 += e * expert_rows;
       }
@@ -1331,7 +1353,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     bool ok = true;
     uint32_t g = 0;  // K blocks issued so far: block g uses accumulator g % 4 for the (g / 4)-th time
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-      if (tile_expert != nullptr && tile_expert[tile % m_tiles] < 0) continue;
+      if (tile_expert != nullptr && tile_expert[tile_m(tile)] < 0) continue;
       for (int kb = 0; kb < k_blocks; ++kb, ++g) {
         const int acc = g & (kFbAcc - 1);
         if (!mbar_wait_warp(tempty_bar(acc), ((g / kFbAcc) & 1) ^ 1, abort_flag)) { ok = false; break; }
@@ -1360,10 +1382,10 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       int e = 0;
       if (tile_expert != nullptr) {
-        e = tile_expert[tile % m_tiles];
+        e = tile_expert[tile_m(tile)];
         if (e < 0) continue;
       }
-      const int m0 = (tile % m_tiles) * kBM, n0 = (tile / m_tiles) * BN;
+      const int m0 = tile_m(tile) * kBM, n0 = tile_n(tile) * BN;
       const int row = m0 + q * 32 + lane;
       const bool row_ok = row < M;
       const float* as = a_scale + (int64_t)(row_ok ? row : 0) * k_blocks;
@@ -1671,6 +1693,20 @@ XLLM_API int xllm_gemm_bf16_grouped_act_mul(const void* a, const void* w, void* 
   mode.act_alpha = alpha;
   if (N % 256 == 0) return launch_gemm<256, 4>(a, w, c, nullptr, M, N, K, lda, K, ldc, 148, 0, s, te, n_experts, mode);
   return launch_gemm<128, 6>(a, w, c, nullptr, M, N, K, lda, K, ldc, 148, 0, s, te, n_experts, mode);
+}
+
+// xllm_gemm_bf16_grouped and (act != 0) xllm_gemm_bf16_grouped_act_mul over row tiles of 256, one CTA pair a tile: two thirds
+// of the operand rows per output of single CTAs.  M and N multiples of 256.
+XLLM_API int xllm_gemm_bf16_grouped_pair(const void* a, const void* w, void* c, const void* tile_expert, int M, int N, int K,
+                                         int n_experts, int64_t lda, int64_t ldc, int act, float limit, float alpha,
+                                         void* stream) {
+  using namespace xllm;
+  if (M == 0 || N == 0) return 0;
+  if (K % 8 || N % 256 || lda % 8 || ldc % 8 || M % (2 * kBM) || act < 0 || act > 4 || tile_expert == nullptr ||
+      (((uintptr_t)a | (uintptr_t)w | (uintptr_t)c) & 15))
+    return (int)cudaErrorInvalidValue;
+  return launch_gemm_pair<256, 6>(a, w, c, nullptr, M, N, K, lda, K, ldc, 148, 0, (cudaStream_t)stream, 1, act, limit, alpha,
+                                  (const int32_t*)tile_expert, n_experts);
 }
 
 // fp8 (e4m3) scaled GEMM: C[M,N] (bf16) = (A_fp8[M,K] · W_fp8[N,K]^T) * a_scale * b_scale (+ bias).

@@ -20,6 +20,7 @@ _lib.register_signature("xllm_moe_offsets", [P, P, P, P, I, I, I, P])
 _lib.register_signature("xllm_moe_offsets_tile", [P, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_moe_permute_fp8", [P, P, P, P, P, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_gemm_bf16_grouped_few", [P, P, P, P, I, I, I, I, I, L, L, I, F, F, P])
+_lib.register_signature("xllm_gemm_bf16_grouped_pair", [P, P, P, P, I, I, I, I, L, L, I, F, F, P])
 _lib.register_signature("xllm_moe_permute", [P, P, P, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_moe_finalize", [P, P, L, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_moe_grouped_simt", [P, P, P, P, I, I, I, L, L, I, P])
@@ -68,13 +69,18 @@ def fused_moe_reference(x, logits, w_gate_up, w_down, top_k, scoring="softmax", 
 
 
 MIN_TILE = 16
+MANY_ROWS = 112          # per expert: from here on, tiles of 256 rows
 
 
 def row_tile(T, top_k, n_experts):
     """Rows of a tile of the grouped products, none of which two experts share.  With few rows per expert the products are
     bound by the experts' weights, and small tiles (csrc/kernels/gemm_few.cu) leave out the rows that are not there; an
     expert with more rows than a tile reads its weights again for the next, from L2.  So: the smallest tile that holds
-    about 2.5 times the average, 128 (gemm_tcgen05.cu) beyond."""
+    about 2.5 times the average, 128 (gemm_tcgen05.cu) beyond.  Many rows are bound by the operands' way from L2: a CTA
+    pair's tile of 256 reads 256 rows of operands per SM and K block for what takes single CTAs' 128-row tiles 384, so it
+    is the better one for experts of more than 128 rows, up to 256 of which it pads to as much as two of the others."""
+    if T * top_k >= MANY_ROWS * n_experts:
+        return 256
     return next((t for t in (16, 32, 64) if T * top_k * 5 <= 2 * t * n_experts), 128)
 
 
@@ -82,7 +88,8 @@ class MoeWorkspace:
     """Static-size buffers of one MoE layer shape (sized for max_tokens; reusable across layers)."""
 
     def __init__(self, max_tokens, top_k, n_experts, n_local, hidden, inter, device, dtype=torch.bfloat16, y_width=None):
-        self.rows = (max_tokens * top_k + n_local * 127 + 127) // 128 * 128
+        widest = 256 if max_tokens * top_k >= MANY_ROWS * n_experts else 128
+        self.rows = (max_tokens * top_k + n_local * (widest - 1) + widest - 1) // widest * widest
         self.max_tiles = self.rows // 128
         i32 = dict(dtype=torch.int32, device=device)
         self.counts = torch.zeros(n_experts, **i32)
@@ -158,9 +165,11 @@ def fused_moe(x, logits, w_gate_up, w_down, top_k, scoring="softmax", bias=None,
                              (0 if scoring == "softmax" else 1) + (2 if group_score == "max" else 0), int(renorm), float(scale), expert_begin, expert_begin + E_local, s), "moe_route")
     simt = w_scales is None and (dt == 1 or H % 8 or I2 % 64 or inter % 8 or Y % 64)
     tile = 128 if simt or I2 % 128 or Y % 128 else row_tile(T, top_k, E)
+    if tile == 256 and (w_scales is not None or I2 % 256 or Y % 256):
+        tile = 128
     # rows that T tokens can take: a workspace is made for more
     rows = min(ws.rows, (T * top_k + min(E_local, T * top_k) * (tile - 1) + tile - 1) // tile * tile)
-    te = ws.tile_expert if tile == 128 else ws.small_tile_expert
+    te = ws.tile_expert if tile >= 128 else ws.small_tile_expert
     check(lib.xllm_moe_offsets_tile(ptr(ws.counts), ptr(ws.offsets), ptr(te), ptr(ws.meta), E, min(te.shape[0], rows // tile),
                                     expert_begin, tile, s), "moe_offsets")
     launches = 6
@@ -190,7 +199,10 @@ def fused_moe(x, logits, w_gate_up, w_down, top_k, scoring="softmax", bias=None,
         product(ws.a, w_down, ws.y)
     elif w_scales is None:
         def grouped(a, w, c, n, k, *glu_args):
-            if tile != 128:
+            if tile == 256:
+                check(lib.xllm_gemm_bf16_grouped_pair(ptr(a), ptr(w), ptr(c), ptr(te), rows, n, k, E_local, k, c.shape[1],
+                                                      *(glu_args or (0, 0.0, 0.0)), s), "moe_gemm_pair")
+            elif tile != 128:
                 check(lib.xllm_gemm_bf16_grouped_few(ptr(a), ptr(w), ptr(c), ptr(te), tile, rows, n, k, E_local, k, c.shape[1],
                                                      *(glu_args or (0, 0.0, 0.0)), s), "moe_gemm_few")
             elif glu_args:
