@@ -51,7 +51,7 @@ struct GdnParams {
 // One warp per (run of rows, item): the heads of q | k | v, then one item for the decays and betas.  A lane owns four
 // neighbouring channels (dk, dv <= 128) and keeps the last inputs in registers, so that every input is read once.
 template <int RUN, int K1>
-__global__ void __launch_bounds__(256) gdn_conv_kernel(GdnParams p) {
+__global__ void __launch_bounds__(256, RUN > 1 ? 3 : 2) gdn_conv_kernel(GdnParams p) {
   const int lane = threadIdx.x & 31, items = 2 * p.G + p.H + 1;
   const unsigned it = blockIdx.x * 8 + (threadIdx.x >> 5), run = it / items;
   pdl_wait();
@@ -97,12 +97,55 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(GdnParams p) {
   for (int t = 0; t < 4; ++t)
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[t][j] = t <= K1 ? __bfloat162float(wr[j * (K1 + 1) + (t <= K1 ? K1 - t : 0)]) : 0.f;
-  int b = -1, begin = 0, end = 0, slot = -1, len = 0;
+  const auto finish = [&](int row, float* s) {
+    float ss = 0.f;
 #pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s[j] = on ? __bfloat162float(__float2bfloat16(silu_as<bf16>(s[j]))) : 0.f;
+      ss += s[j] * s[j];
+    }
+    if (part < 2) {
+      ss = warp_sum(ss);
+      if (lane == 0) (part == 0 ? p.fq : p.fk)[(int64_t)row * p.G + h] = (part == 0 ? p.q_scale : 1.f) * rsqrtf(ss + kGdnUnitEps);
+    }
+    if (c < dp) store_f32<4>(y + row * y_ld, s);                     // zeros behind d
+  };
+  int b = seq_of_row(p.cu_q, p.n_seqs, first), begin = first, end = first + 1, slot = -1, len = 0;
+  if (b >= 0) {
+    begin = p.cu_q[b];
+    end = p.cu_q[b + 1];
+    slot = p.slots[b];
+    len = p.kv_lens[b];
+  }
+  if (RUN > 1 && slot >= 0 && first - begin >= K1 && first + RUN <= end) {      // most runs: no edge of a sequence nearby
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+      float s[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[j] = v[i + 3][j] * w[0][j];
+#pragma unroll
+        for (int t = 1; t <= K1; ++t) s[j] += v[i + 3 - t][j] * w[t][j];
+      }
+      finish(first + i, s);
+    }
+    return;
+  }
+#pragma unroll 1
   for (int i = 0; i < RUN; ++i) {
     const int row = first + i;
     if (row >= p.rows) break;
-    if (row >= end) {                                               // the row starts another sequence, or is the first
+    float x0[4][4];                                                 // x0[t]: t rows back
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x0[t][j] = 0.f;
+#pragma unroll
+        for (int u = 0; u < RUN; ++u)
+          if (u == i) x0[t][j] = v[u + 3 - t][j];
+      }
+    if (row >= end) {                                               // the row starts another sequence
       b = seq_of_row(p.cu_q, p.n_seqs, row);
       begin = b < 0 ? row : p.cu_q[b];
       end = b < 0 ? row + 1 : p.cu_q[b + 1];
@@ -114,18 +157,18 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(GdnParams p) {
     float s[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      s[j] = v[i + 3][j] * w[0][j];
-      if (back >= 1) s[j] += v[i + 2][j] * w[1][j];
-      if (back >= 2) s[j] += v[i + 1][j] * w[2][j];
-      if (back >= 3) s[j] += v[i][j] * w[3][j];
+      s[j] = x0[0][j] * w[0][j];
+      if (back >= 1) s[j] += x0[1][j] * w[1][j];
+      if (back >= 2) s[j] += x0[2][j] * w[2][j];
+      if (back >= 3) s[j] += x0[3][j] * w[3][j];
     }
     bf16* tail = p.tail + ((int64_t)slot * C + ch) * K1;            // [channel][input], oldest first
     if (back < K1 && on) {
       __align__(8) bf16 past[4 * K1];
       const bool old = len > n;                                     // the slot's tail belongs to this sequence
 #pragma unroll
-      for (int i = 0; i < K1; ++i)
-        *reinterpret_cast<uint2*>(past + 4 * i) = old ? reinterpret_cast<const uint2*>(tail)[i] : make_uint2(0u, 0u);
+      for (int q = 0; q < K1; ++q)
+        *reinterpret_cast<uint2*>(past + 4 * q) = old ? reinterpret_cast<const uint2*>(tail)[q] : make_uint2(0u, 0u);
 #pragma unroll
       for (int u = 0; u < K1; ++u) {                                // u + 1 inputs before the sequence's rows
         const int t = u + 1 + back;
@@ -138,22 +181,12 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(GdnParams p) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
-          for (int t = 0; t < K1; ++t) now[j * K1 + t] = t + 1 < K1 ? past[j * K1 + t + 1] : __float2bfloat16(v[i + 3][j]);
+          for (int t = 0; t < K1; ++t) now[j * K1 + t] = t + 1 < K1 ? past[j * K1 + t + 1] : __float2bfloat16(x0[0][j]);
 #pragma unroll
-        for (int i2 = 0; i2 < K1; ++i2) reinterpret_cast<uint2*>(tail)[i2] = *reinterpret_cast<const uint2*>(now + 4 * i2);
+        for (int q = 0; q < K1; ++q) reinterpret_cast<uint2*>(tail)[q] = *reinterpret_cast<const uint2*>(now + 4 * q);
       }
     }
-    float ss = 0.f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      s[j] = on ? __bfloat162float(__float2bfloat16(silu_as<bf16>(s[j]))) : 0.f;
-      ss += s[j] * s[j];
-    }
-    if (part < 2) {
-      ss = warp_sum(ss);
-      if (lane == 0) (part == 0 ? p.fq : p.fk)[(int64_t)row * p.G + h] = (part == 0 ? p.q_scale : 1.f) / sqrtf(ss + kGdnUnitEps);
-    }
-    if (c < dp) store_f32<4>(y + row * y_ld, s);                     // zeros behind d
+    finish(row, s);
   }
 }
 
@@ -647,14 +680,14 @@ XLLM_API int xllm_gdn_layer(void* state, void* tail, const void* slots, const vo
   p.n_decode = n_decode; p.n_seqs = n_seqs; p.rows = rows; p.H = H; p.G = G; p.dk = dk; p.dv = dv; p.taps = taps;
   p.q_scale = q_scale; p.eps = eps;
   cudaStream_t s = (cudaStream_t)stream;
-  // runs of eight rows read eleven inputs of a channel where eight single rows read 32; few rows need the warps more than
-  // the reuse
-  const int items = 2 * G + H + 1, run = rows > 128 ? 8 : 1;
+  // Runs of four rows read seven inputs of a channel where four single rows read sixteen; few rows need the warps more than
+  // the reuse.  Bound by latency and instructions: the registers of longer runs cost more in warps than their reuse gives.
+  const int items = 2 * G + H + 1, run = rows > 128 ? 4 : 1;
   const dim3 grid((unsigned)((((int64_t)rows + run - 1) / run * items + 7) / 8));
   const auto conv = [&](auto kernel) { launch_pdl(kernel, grid, dim3(256), 0, s, p); };
-  if (taps == 4) conv(run > 1 ? gdn_conv_kernel<8, 3> : gdn_conv_kernel<1, 3>);
-  else if (taps == 3) conv(run > 1 ? gdn_conv_kernel<8, 2> : gdn_conv_kernel<1, 2>);
-  else conv(run > 1 ? gdn_conv_kernel<8, 1> : gdn_conv_kernel<1, 1>);
+  if (taps == 4) conv(run > 1 ? gdn_conv_kernel<4, 3> : gdn_conv_kernel<1, 3>);
+  else if (taps == 3) conv(run > 1 ? gdn_conv_kernel<4, 2> : gdn_conv_kernel<1, 2>);
+  else conv(run > 1 ? gdn_conv_kernel<4, 1> : gdn_conv_kernel<1, 1>);
   int rc = XLLM_LAUNCH_CHECK();
   if (rc != 0) return rc;
   if (n_seqs > n_decode) {

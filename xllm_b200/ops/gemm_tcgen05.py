@@ -11,6 +11,7 @@ from ._lib import F, I, L, P, check, ptr, stream
 
 _lib.register_signature("xllm_gemm_bf16", [P, P, P, P, I, I, I, L, L, L, I, I, I, I, P])
 _lib.register_signature("xllm_gemm_error_status", [], I)
+_lib.register_signature("xllm_gemm_few_error_status", [], I)
 _lib.register_signature("xllm_gemm_prepare", [], I)
 _lib.register_signature("xllm_gemm_set_k_per_stage", [I], None)
 _lib.register_signature("xllm_gemm_set_dual_issue", [I], None)
@@ -176,4 +177,5 @@ def prepare():
 
 def error_status() -> int:
     """Non-zero when a bounded wait inside a GEMM kernel expired since the last query."""
-    return int(_lib.load().xllm_gemm_error_status())
+    lib = _lib.load()
+    return int(lib.xllm_gemm_error_status()) | int(lib.xllm_gemm_few_error_status())
