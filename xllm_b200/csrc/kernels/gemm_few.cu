@@ -144,8 +144,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
       const int st = i % S::stages;
       if (!mbar_wait_warp(empty(st), ((i / S::stages) & 1) ^ 1, abort_flag)) { ok = false; break; }
-      if (lane == 0) {
-        const uint32_t dst = sbase + st * S::stage;
+      const uint32_t dst = sbase + st * S::stage;
+      if (elect_one()) {
         mbar_expect_tx(full(st), S::w_bytes + p.x_rows * 128);
         tma_load_2d(dst, &tma_w, kb * KE, wy, full(st));
         tma_load_2d(dst + S::w_bytes, &tma_x, kb * KE, m0, full(st));
@@ -164,13 +164,12 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       if (FP8 && !mbar_wait_warp(tempty(a), ((i / kAcc) & 1) ^ 1, abort_flag)) break;
       if (!mbar_wait_warp(full(st), (i / S::stages) & 1, abort_flag)) break;
       tc_fence_after();
-      if (lane == 0) {
-        const uint32_t w = sbase + st * S::stage, x = w + S::w_bytes;
+      const uint64_t wd = smem_desc(sbase + st * S::stage, 16, 1024), xd = smem_desc(sbase + st * S::stage + S::w_bytes, 16, 1024);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint64_t wd = smem_desc(w + k * 32, 16, 1024), xd = smem_desc(x + k * 32, 16, 1024);
-          if constexpr (FP8) umma_fp8(tmem + a * TN, wd, xd, ID, k != 0);
-          else umma(tmem, wd, xd, ID, (i | k) != 0);
+          if constexpr (FP8) umma_fp8(tmem + a * TN, wd + 2 * k, xd + 2 * k, ID, k != 0);
+          else umma(tmem, wd + 2 * k, xd + 2 * k, ID, (i | k) != 0);
         }
         umma_commit(empty(st));        // the ring slot is free once these MMAs have read it
         if (FP8) umma_commit(tfull(a));                // ... and the block's product is complete
