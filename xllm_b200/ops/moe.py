@@ -78,7 +78,9 @@ def row_tile(T, top_k, n_experts):
     expert with more rows than a tile reads its weights again for the next, from L2.  So: the smallest tile that holds
     about 2.5 times the average, 128 (gemm_tcgen05.cu) beyond.  Many rows are bound by the operands' way from L2: a CTA
     pair's tile of 256 reads 256 rows of operands per SM and K block for what takes single CTAs' 128-row tiles 384, so it
-    is the better one for experts of more than 128 rows, up to 256 of which it pads to as much as two of the others."""
+    is the better one for experts of more than 128 rows, up to 256 of which it pads to as much as two of the others.
+    Measured (one B200, 128 experts of 768, a layer's two products): 16 tokens 189 us in tiles of 128, 126 us in tiles of
+    16; 3066 tokens (192 rows per expert) 306 us in tiles of 128, 285 us in pairs' tiles of 256."""
     if T * top_k >= MANY_ROWS * n_experts:
         return 256
     return next((t for t in (16, 32, 64) if T * top_k * 5 <= 2 * t * n_experts), 128)
