@@ -14,7 +14,8 @@
 //
 // Measured against the same layer as tensor operations around gdn.cu (one B200, 32 heads of 128 x 128, four prompts of up to
 // 1024 tokens one after the other: 3.6 ms a layer; 64 decode rows: 0.55 ms), whose time went to some fifty launches of
-// elementwise kernels, the prompts one by one, and two barriers per token in the recurrence.
+// elementwise kernels, the prompts one by one, and two barriers per token in the recurrence.  Now 0.31 ms (convolution 60 us,
+// chunks 20 and 198 us, norm 34 us) and 0.06 ms, of which the step takes 48 us (states: 268 MB, 41 us at the copy rate).
 //
 // A sequence whose rows in the batch are its first tokens (kv_len == number of rows) starts from zeros whatever its slot
 // holds; slot < 0 marks padding rows, which come out as zeros.  Built without fast-math: errors of a decay multiply up.
@@ -291,7 +292,8 @@ __global__ void __launch_bounds__(256, 2) gdn_step_kernel(GdnParams p) {
 // without leaving the registers, as U^T is of the products behind it.
 //
 // Token by token in fp32 (states in registers, no barriers) the walk took 600 us for four prompts of 1024, 549, 842 and 366
-// tokens, 32 heads of 128 x 128 (one B200), some 1100 cycles a token in a chain of product, exchange, product.
+// tokens, 32 heads of 128 x 128 (one B200), some 1100 cycles a token in a chain of product, exchange, product; in chunks it
+// takes 198 us, the preparation 20 us.
 constexpr int kGC = 16, kGWarps = 4, kGCols = 16 * kGWarps, kGStages = 3, kGVld = kGCols + 8;
 
 struct GdnBlob {                             // bytes of one (chunk, head)
@@ -325,7 +327,8 @@ template <int DK>
 __global__ void __launch_bounds__(128) gdn_prep_kernel(GdnParams p) {
   constexpr int LD = DK + 8, PC = DK / 8;
   __shared__ __align__(16) bf16 rows[2][kGC][LD];                    // k, q
-  __shared__ float dots[2][kGC][kGC + 1], am[4][kGC][kGC + 1], gs[4][kGC], bs[4][kGC], ff[2][kGC];
+  __shared__ float dots[2][kGC][kGC + 1], am[4][kGC][kGC + 1], bs[4][kGC], ff[2][kGC];
+  __shared__ double gs[4][kGC];                                      // sums of g: differences of large ones must not lose the small
   const int g = blockIdx.y, b = p.n_decode + blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_wait();
   pdl_launch_dependents();
@@ -362,7 +365,7 @@ __global__ void __launch_bounds__(128) gdn_prep_kernel(GdnParams p) {
   for (int i = warp; i < r; i += 4) {
     const int h = g * r + i;
     uint8_t* blob = p.blobs + (gdn_chunk_slot(first, blockIdx.z, blockIdx.x) * p.H + h) * GdnBlob::bytes;
-    float G = 0.f;
+    double G = 0.;
     if (lane < kGC) {
       const float2 gb = lane < n ? p.gb[(int64_t)(row0 + lane) * p.H + h] : make_float2(0.f, 0.f);
       G = gb.x;                                                      // g: rows behind the last one add nothing
@@ -370,20 +373,20 @@ __global__ void __launch_bounds__(128) gdn_prep_kernel(GdnParams p) {
     }
 #pragma unroll
     for (int o = 1; o < kGC; o <<= 1) {
-      const float x = __shfl_up_sync(0xffffffffu, G, o);
+      const double x = __shfl_up_sync(0xffffffffu, G, o);
       if (lane >= o) G += x;
     }
-    const float end = __shfl_sync(0xffffffffu, G, kGC - 1);
+    const double end = __shfl_sync(0xffffffffu, G, kGC - 1);
     if (lane < kGC) {
       gs[warp][lane] = G;
-      const float e = expf(G);
+      const float e = expf((float)G);
       reinterpret_cast<float4*>(blob + GdnBlob::f)[lane] =
-          make_float4(ff[0][lane] * e, ff[1][lane] * e, ff[0][lane] * expf(end - G), expf(end));
+          make_float4(ff[0][lane] * e, ff[1][lane] * e, ff[0][lane] * expf((float)(end - G)), expf((float)end));
     }
     __syncwarp();
     for (int x = lane; x < kGC * kGC; x += 32) {
       const int t = x >> 4, s = x & 15;
-      const float e = s <= t ? expf(gs[warp][t] - gs[warp][s]) * ff[0][s] : 0.f;
+      const float e = s <= t ? expf((float)(gs[warp][t] - gs[warp][s])) * ff[0][s] : 0.f;
       am[warp][t][s] = s < t ? bs[warp][t] * ff[0][t] * e * dots[0][t][s] : 0.f;
       put3(reinterpret_cast<bf16*>(blob + GdnBlob::p) + x, kGC * kGC, ff[1][t] * e * dots[1][t][s]);
     }
