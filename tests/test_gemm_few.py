@@ -57,6 +57,31 @@ def test_fp8_pairs(M, N, K):
     test_fp8(M, N, K)
 
 
+# every tile that the numbers of rows and columns choose, with K blocks that fill no stage, one slice and more of a ring, and a K
+# whose scales are too many for them
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("N,K", [(8, 128), (576, 7168), (1544, 384), (6400, 640), (7168, 2048), (12800, 256), (25608, 384), (128, 49280)])
+def test_fp8_rows_do_not_depend_on_their_number(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M * N + K)
+    a, a_s = fp8.quant_group128(torch.randn(130, K, device=DEV, generator=g).bfloat16())
+    w, w_s = fp8.quant_block128_ref(torch.randn(N, K, device=DEV, generator=g))
+    assert torch.equal(fp8.block_scaled_mm(a[:M], a_s[:M], w, w_s), fp8.block_scaled_mm(a, a_s, w, w_s)[:M])
+
+
+@pytest.mark.parametrize("tile", [16, 32, 64])
+@pytest.mark.parametrize("N,K", [(128, 128), (384, 640), (512, 1152)])
+def test_fp8_experts_rows_do_not_depend_on_the_tile(tile, N, K):
+    g = torch.Generator(device=DEV).manual_seed(tile + K)
+    a, a_s = fp8.quant_group128(torch.randn(256, K, device=DEV, generator=g).bfloat16())
+    parts = [fp8.quant_block128_ref(torch.randn(N, K, device=DEV, generator=g)) for _ in range(2)]
+    w, w_s = torch.stack([p[0] for p in parts]), torch.stack([p[1] for p in parts])
+    large, small = (torch.empty(256, N, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    experts = torch.tensor([1, 0], dtype=torch.int32, device=DEV)
+    fp8.block_scaled_mm_grouped(a, a_s, w, w_s, experts, large, 128)
+    fp8.block_scaled_mm_grouped(a, a_s, w, w_s, experts.repeat_interleave(128 // tile), small, tile)
+    assert torch.equal(large, small)
+
+
 @pytest.mark.parametrize("tile", [16, 32, 64, 256])
 @pytest.mark.parametrize("kind", ["bf16", "gated", "fp8"])
 def test_grouped(tile, kind):

@@ -9,13 +9,19 @@
 // The operands are swapped: 128 WEIGHT rows are the rows of the tcgen05 tile and 16, 32 or 64 token rows its columns, so what
 // is read back (per K block for fp8, whose blocks differ in scale) is the tokens there are, not 128 columns of weights for a
 // tile of mostly absent rows, and an expert with four rows costs no loads and stores of 128.  A CTA needs half an SM, and two
-// of them cover each other's start and end.  Where the tiles alone leave SMs idle, a cluster of up to eight CTAs cuts K:
-// every CTA sums its slice, the slices meet through distributed shared memory, in a fixed order.  (Split-K in
-// gemm_tcgen05.cu meets in scratch memory by reduce-adds, a round trip of some 6 us.)  The first weights of an ungrouped
-// product start for L2 before the wait for the kernel in front.
+// of them cover each other's start and end.  The first weights of an ungrouped product start for L2 before the wait for the
+// kernel in front.  Where the tiles alone leave SMs idle:
+//
+//   bf16  a cluster of up to eight CTAs cuts K: every CTA sums its slice, the slices meet through distributed shared memory, in a
+//         fixed order.  (Split-K in gemm_tcgen05.cu meets in scratch memory by reduce-adds, a round trip of some 6 us.)
+//   fp8   narrower tiles, of 64 or 32 weight rows (instructions of 64 rows; of 32 weight rows, the others are whatever lies behind
+//         and are not read back), and more of them side by side for more rows of A.  K stays whole, so that the scaled blocks
+//         are added one after the other as in gemm_fp8_block_kernel and a row comes out with the same bits however many rows
+//         there are: the e4m3 rounding in front of the next product turns other last bits into other values (K cut over
+//         clusters: a step of two latent layers 0.02 to 0.03 from the same rows' among many).
 //
 // Measured (one B200, 16 rows, before: gemm_fp8_block_kernel): 7168 x 16384 fp8 (117 MB of weights, 18 us at the copy rate)
-// 55 -> 27 us, 1536 x 7168 24 -> 7 us, 7168 x 18432 58 -> 26 us; 32 experts' 4096 x 7168 and 7168 x 2048 fp8 190 -> 126 us and
+// 56 -> 29 us, 1536 x 7168 25 -> 10 us, 7168 x 18432 63 -> 32 us; 32 experts' 4096 x 7168 and 7168 x 2048 fp8 190 -> 126 us and
 // 210 -> 63 us.  bf16, one row (before: split-K in gemm_tcgen05.cu, and the activation's own kernel): 4096 x 4096 13 -> 9 us,
 // gated 24576 x 4096 44 -> 39 us (31 at the copy rate), 4096 x 12288 26 -> 20 us.
 //
@@ -29,16 +35,23 @@ namespace few {
 
 using namespace tc;
 
-constexpr int kAcc = 4, kMaxSplit = 8, kPrefetchBlocks = 8;
+constexpr int kMaxSplit = 8, kPrefetchBlocks = 8;
+constexpr int kFp8MaxK = 49152;        // the scales of a whole K lie in shared memory: 98 KB at most
 
-template <int TN, bool FP8>
+// WR: weight rows of a tile; G: K blocks of a stage of the ring, which are also read back together
+template <int TN, bool FP8, int WR, int G>
 struct Smem {
-  static constexpr int cols = FP8 ? kAcc * TN : (TN < 32 ? 32 : TN);   // of tensor memory
-  static constexpr int stages = TN == 64 ? 3 : 4;
-  static constexpr int w_bytes = 128 * 128, x_bytes = TN * 128, stage = w_bytes + x_bytes;
-  static constexpr int bars = stages * stage, scales = bars + (2 * stages + 2 * kAcc) * 8 + 16;
-  static constexpr int total(int k_blocks) { return scales + (FP8 ? k_blocks * TN * 4 : 0) + 1024; }
-  static_assert(stage % 1024 == 0 && 2 * TN * 128 * 4 <= stages * stage, "the sums meet where the ring was");
+  static constexpr int acc = FP8 ? (256 / (G * TN) < 4 ? 256 / (G * TN) : 4) : 1;     // groups of G accumulators
+  static constexpr int cols = FP8 ? acc * G * TN : (TN < 32 ? 32 : TN);               // of tensor memory
+  static constexpr int w_bytes = WR * 128, x_bytes = TN * 128, block = w_bytes + x_bytes, stage = G * block;
+  static constexpr int stages = FP8 ? 100 * 1024 / stage : (TN == 64 ? 3 : 4);
+  static constexpr int rows = WR < 128 ? 64 : 128;                                    // of an instruction
+  static constexpr int behind = rows * 128 - block > 0 ? rows * 128 - block : 0;      // rows the last block's instructions read beyond it
+  static constexpr int readers = WR < 128 ? WR / 16 : 4;                              // warps with rows of the tile
+  static constexpr int bars = stages * stage + behind, scales = bars + (2 * stages + 2 * acc) * 8 + 16;
+  static constexpr int total(int k_blocks) { return scales + (FP8 ? k_blocks * (TN + 1) * 4 : 0) + 1024; }
+  static_assert(WR % 32 == 0 && block % 1024 == 0 && cols <= 256 && acc >= 2 - !FP8, "swizzled tiles, and two CTAs an SM");
+  static_assert(FP8 || (WR == 128 && G == 1 && 2 * TN * 128 * 4 <= stages * stage), "the sums meet where the ring was");
 };
 
 struct Params {
@@ -74,6 +87,10 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr, uint32_t rank) {
   return v;
 }
 
+__device__ __forceinline__ void copy_f32(float* dst, const float* src, bool in) {      // zero where not
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+
 __device__ __forceinline__ float gated(float x, float y, int act, float limit, float alpha) {
   if (act == 4) return clamped_glu(x, y, limit, alpha);
   if (act == 1) return x / (1.f + __expf(-x)) * y;
@@ -81,11 +98,12 @@ __device__ __forceinline__ float gated(float x, float y, int act, float limit, f
   return 0.5f * x * (1.f + tanhf(0.7978845608f * (x + 0.044715f * x * x * x))) * y;
 }
 
-// grid (slices of K = the cluster, row tiles x tiles of 128 weight rows)
-template <int TN, bool FP8>
+// grid (slices of K = the cluster, row tiles x tiles of WR weight rows)
+template <int TN, bool FP8, int WR, int G>
 __global__ void __launch_bounds__(192, 2)
 gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w, const Params p) {
-  using S = Smem<TN, FP8>;
+  using S = Smem<TN, FP8, WR, G>;
+  constexpr int kAcc = S::acc;
   constexpr int KE = FP8 ? 128 : 64;                                  // elements of a K block
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -109,13 +127,13 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     }
     for (int a = 0; a < kAcc; ++a) {
       mbar_init(tfull(a), 1);
-      mbar_init(tempty(a), 4);
+      mbar_init(tempty(a), S::readers);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (p.tile_expert == nullptr && warp == 0) {
-    if (lane < kPrefetchBlocks && kb0 + lane < kb1) prefetch_2d(&tma_w, (kb0 + lane) * KE, nt * 128);
+    if (lane < kPrefetchBlocks && kb0 + lane < kb1) prefetch_2d(&tma_w, (kb0 + lane) * KE, nt * WR);
     __syncwarp();
   }
   pdl_wait();
@@ -133,7 +151,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_holder;
-  const int m0 = mt * TN, n0 = nt * 128;
+  const int m0 = mt * TN, n0 = nt * WR;
   const int live = min(TN, p.M - m0);
   float acc[TN];
   bool ok = true;
@@ -141,14 +159,18 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     const int wy = expert * p.N + n0;
-    for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+    for (int kb = kb0, i = 0; kb < kb1; kb += G, ++i) {
       const int st = i % S::stages;
       if (!mbar_wait_warp(empty(st), ((i / S::stages) & 1) ^ 1, abort_flag)) { ok = false; break; }
       const uint32_t dst = sbase + st * S::stage;
       if (elect_one()) {
-        mbar_expect_tx(full(st), S::w_bytes + p.x_rows * 128);
-        tma_load_2d(dst, &tma_w, kb * KE, wy, full(st));
-        tma_load_2d(dst + S::w_bytes, &tma_x, kb * KE, m0, full(st));
+        mbar_expect_tx(full(st), min(G, kb1 - kb) * (S::w_bytes + p.x_rows * 128));
+#pragma unroll
+        for (int b = 0; b < G; ++b)
+          if (kb + b < kb1) {
+            tma_load_2d(dst + b * S::block, &tma_w, (kb + b) * KE, wy, full(st));
+            tma_load_2d(dst + b * S::block + S::w_bytes, &tma_x, (kb + b) * KE, m0, full(st));
+          }
       }
       __syncwarp();
     }
@@ -158,21 +180,26 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    constexpr uint32_t ID = FP8 ? (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24) : idesc(false, TN);
-    for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+    constexpr uint32_t ID = FP8 ? (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(S::rows >> 4) << 24) : idesc(false, TN);
+    for (int kb = kb0, i = 0; kb < kb1; kb += G, ++i) {
       const int st = i % S::stages, a = i % kAcc;
       if (FP8 && !mbar_wait_warp(tempty(a), ((i / kAcc) & 1) ^ 1, abort_flag)) break;
       if (!mbar_wait_warp(full(st), (i / S::stages) & 1, abort_flag)) break;
       tc_fence_after();
       const uint64_t wd = smem_desc(sbase + st * S::stage, 16, 1024), xd = smem_desc(sbase + st * S::stage + S::w_bytes, 16, 1024);
       if (elect_one()) {
+        // the blocks of a stage in turn: a product waits for the one in front that adds to the same accumulator
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if constexpr (FP8) umma_fp8(tmem + a * TN, wd + 2 * k, xd + 2 * k, ID, k != 0);
-          else umma(tmem, wd + 2 * k, xd + 2 * k, ID, (i | k) != 0);
-        }
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int b = 0; b < G; ++b)
+            if (G == 1 || kb + b < kb1) {
+              const uint64_t at = b * (S::block >> 4) + 2 * k;
+              if constexpr (FP8) umma_fp8(tmem + (a * G + b) * TN, wd + at, xd + at, ID, k != 0);
+              else umma(tmem, wd + at, xd + at, ID, (i | k) != 0);
+            }
         umma_commit(empty(st));        // the ring slot is free once these MMAs have read it
-        if (FP8) umma_commit(tfull(a));                // ... and the block's product is complete
+        if (FP8) umma_commit(tfull(a));                // ... and the blocks' products are complete
         else if (kb + 1 == kb1) umma_commit(tfull(0));
       }
       __syncwarp();
@@ -183,37 +210,61 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     constexpr int C = TN < 32 ? 16 : 32;
     if constexpr (FP8) {
+      // All of them in flight together, then each times its block's: a load at a time, they took longer than the weights.
       const float* ws = p.w_scale + ((int64_t)expert * p.N + n0) / 128 * p.k_blocks + kb0;
-      for (int i = t; i < n_kb * TN; i += 128) {
-        const int r = i / n_kb, k = i - r * n_kb;
-        scales[k * TN + r] = r < live ? p.a_scale[(int64_t)(m0 + r) * p.k_blocks + kb0 + k] * ws[k] : 0.f;
+      const int at_k = n_kb * TN;                       // the weights' scales lie behind the rows'
+      for (int r = warp - 2; r < TN; r += 4)
+        for (int k = lane; k < n_kb; k += 32)
+          copy_f32(scales + k * TN + r, p.a_scale + (int64_t)(m0 + (r < live ? r : 0)) * p.k_blocks + kb0 + k, r < live);
+      for (int k = t; k < n_kb; k += 128) copy_f32(scales + at_k + k, ws + k, true);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      for (int i = t; i < at_k / 4; i += 128) {
+        float4* v = reinterpret_cast<float4*>(scales) + i;
+        const float f = scales[at_k + i / (TN / 4)];
+        float4 x = *v;
+        x.x *= f; x.y *= f; x.z *= f; x.w *= f;
+        *v = x;
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
       for (int j = 0; j < TN; ++j) acc[j] = 0.f;
-      for (int i = 0; i < n_kb; ++i) {
+      const int groups = (warp & 3) < S::readers ? (n_kb + G - 1) / G : 0;
+      constexpr int B = G * TN <= 64 ? G : 1;                                   // blocks read at a time
+      for (int i = 0; i < groups; ++i) {
         const int a = i % kAcc;
         ok = ok && mbar_wait(tfull(a), (i / kAcc) & 1, abort_flag);
         __syncwarp();
         tc_fence_after();
-        uint32_t r[TN];
 #pragma unroll
-        for (int j = 0; j < TN; j += C) {
-          if constexpr (C == 16) tmem_ld16(at + a * TN + j, r + j);
-          else tmem_ld32(at + a * TN + j, r + j);
-        }
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(tempty(a));        // handed back before the arithmetic
-        const float4* sc = reinterpret_cast<const float4*>(scales + i * TN);
+        for (int b0 = 0; b0 < G; b0 += B) {
+          if (G > 1 && i * G + b0 >= n_kb) break;
+          uint32_t r[B * TN];
 #pragma unroll
-        for (int j = 0; j < TN; j += 4) {
-          const float4 f = sc[j >> 2];
-          acc[j] = fmaf(__uint_as_float(r[j]), f.x, acc[j]);
-          acc[j + 1] = fmaf(__uint_as_float(r[j + 1]), f.y, acc[j + 1]);
-          acc[j + 2] = fmaf(__uint_as_float(r[j + 2]), f.z, acc[j + 2]);
-          acc[j + 3] = fmaf(__uint_as_float(r[j + 3]), f.w, acc[j + 3]);
+          for (int j = 0; j < B * TN; j += C) {          // (of blocks behind the last one: what is there, and not used)
+            if constexpr (C == 16) tmem_ld16(at + (a * G + b0) * TN + j, r + j);
+            else tmem_ld32(at + (a * G + b0) * TN + j, r + j);
+          }
+          tmem_ld_wait();
+          if (b0 + B >= G || i * G + b0 + B >= n_kb) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty(a));       // handed back before the arithmetic
+          }
+#pragma unroll
+          for (int b = 0; b < B; ++b) {
+            if (B > 1 && i * G + b >= n_kb) break;
+            const float4* sc = reinterpret_cast<const float4*>(scales + (i * G + b0 + b) * TN);
+            const uint32_t* v = r + b * TN;
+#pragma unroll
+            for (int j = 0; j < TN; j += 4) {
+              const float4 f = sc[j >> 2];
+              acc[j] = fmaf(__uint_as_float(v[j]), f.x, acc[j]);
+              acc[j + 1] = fmaf(__uint_as_float(v[j + 1]), f.y, acc[j + 1]);
+              acc[j + 2] = fmaf(__uint_as_float(v[j + 2]), f.z, acc[j + 2]);
+              acc[j + 3] = fmaf(__uint_as_float(v[j + 3]), f.w, acc[j + 3]);
+            }
+          }
         }
       }
     } else {
@@ -231,12 +282,13 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
       for (int j = 0; j < TN; ++j) acc[j] = __uint_as_float(r[j]);
     }
   }
-  const int row = (warp & 3) * 32 + lane;             // warps 2..5: tensor memory lane = weight row of the tile
-  const bool stores = warp >= 2 && n0 + row < p.N;
+  // warps 2..5: the weight row of the tile at this tensor memory lane (of instructions of 64 rows, 16 lie in every 32 lanes)
+  const int row = S::rows == 128 ? (warp & 3) * 32 + lane : (lane < 16 ? (warp & 3) * 16 + lane : WR);
+  const bool stores = warp >= 2 && row < WR && n0 + row < p.N;
   const float bias = !FP8 && stores && p.bias != nullptr ? __bfloat162float(p.bias[n0 + row]) : 0.f;
   float* red = reinterpret_cast<float*>(smem);        // [row of A][weight row]: every copy of the ring has been consumed
   float* fin = splits > 1 ? red + TN * 128 : red;     // what the activation reads
-  if (splits == 1) {
+  if (FP8 || splits == 1) {
     if (!FP8 && p.act != 0) {
       if (warp >= 2) {
 #pragma unroll
@@ -262,7 +314,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         for (int s = 0; s < kMaxSplit; ++s) v[s] = s < splits ? ld_cluster(at, s) : 0.f;
 #pragma unroll
         for (int s = 0; s < kMaxSplit; ++s) sum += v[s];
-        if (!FP8 && p.act != 0) fin[j * 128 + row] = sum;
+        if (p.act != 0) fin[j * 128 + row] = sum;
         else if (stores && ok) p.c[(int64_t)(m0 + j) * p.ldc + n0 + row] = __float2bfloat16(sum + bias);
       }
     __syncwarp();
@@ -276,7 +328,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
         p.c[(int64_t)(m0 + j) * p.ldc + nt * 64 + f] =
             __float2bfloat16(gated(rounded(fin[j * 128 + f]), rounded(fin[j * 128 + 64 + f]), p.act, p.limit, p.alpha));
   }
-  if (splits > 1) cluster_sync();                     // nobody leaves while its sums are being read
+  if (!FP8 && splits > 1) cluster_sync();             // nobody leaves while its sums are being read
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag && p.err != nullptr) atomicExch(p.err, 1);
@@ -314,24 +366,24 @@ static int choose_split(int tiles, int k_blocks) {
   return best;
 }
 
-template <int TN, bool FP8>
+template <int TN, bool FP8, int WR, int G>
 static int launch(const void* a, const void* w, const Params& p, int K, int64_t lda, int64_t ldw, int n_experts, int splits,
                   int dev, cudaStream_t s) {
-  using S = Smem<TN, FP8>;
+  using S = Smem<TN, FP8, WR, G>;
   static std::atomic<int> attr_bytes[64] = {};
   const int per = (p.k_blocks + splits - 1) / splits, smem = S::total(per);
   if (smem > 232448) return (int)cudaErrorInvalidValue;
   if (attr_bytes[dev & 63].load(std::memory_order_acquire) < smem) {
     // once and for all sizes: a kernel may use what its launch asks for, up to this
-    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<TN, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<TN, FP8, WR, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
     if (e != cudaSuccess) return (int)e;
     attr_bytes[dev & 63].store(232448, std::memory_order_release);
   }
   CUtensorMap tx, tw;
-  if (!make_map_of(&tx, a, p.M, K, lda, p.x_rows, FP8) || !make_map_of(&tw, w, (int64_t)p.N * n_experts, K, ldw, 128, FP8))
+  if (!make_map_of(&tx, a, p.M, K, lda, p.x_rows, FP8) || !make_map_of(&tw, w, (int64_t)p.N * n_experts, K, ldw, WR, FP8))
     return (int)cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, (unsigned)(((p.M + TN - 1) / TN) * ((p.N + 127) / 128)));
+  cfg.gridDim = dim3(splits, (unsigned)(((p.M + TN - 1) / TN) * ((p.N + WR - 1) / WR)));
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -343,20 +395,44 @@ static int launch(const void* a, const void* w, const Params& p, int K, int64_t 
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_few_kernel<TN, FP8>, tx, tw, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_few_kernel<TN, FP8, WR, G>, tx, tw, p);
   return e != cudaSuccess ? (int)e : XLLM_LAUNCH_CHECK();
 }
 
-// tile: rows of A at a time.  Grouped: every tile belongs to one expert, M a multiple of it.
+// Tile of an ungrouped fp8 product, {rows of A, weight rows}: the smallest of which an SM has one or, here and there, two.  A CTA
+// goes through K block by block, and a block takes it what the instructions need (some 170 ns of 128 weight rows, 85 ns of 64 or
+// fewer) or what its sums take to read back (some 65 ns per 16 rows of A, 32 at a time and lane quarter), whichever is longer,
+// while the weights' way from HBM only counts from two thirds of the SMs on.  Measured (one B200, us; 16, 32, 64 rows of A):
+//   {16, 32}   1536 x 7168 10, 10, 13   4096 x 7168 11, 14, 25   7168 x 16384 28, 50, 91
+//   {16, 64}               13, 13, 13               13, 14, 18                29, 36, 66   12288 x 4096 14, 20, 32
+//   {32, 64}                   15, 15                   15, 16                    33, 62                    15, 22
+//   {32, 128}                  19, 19                   20, 20                    46, 45                    16, 17   24576 x 1536 11, 17
+//   {64, 128}                      26                       27                        55                        19           11, 14
+static void fp8_tile(int M, int N, int& tile, int& wr) {
+  constexpr int kTiles = 200;
+  const auto count = [&](int t, int w) { return (int64_t)((M + t - 1) / t) * ((N + w - 1) / w); };
+  tile = 16;
+  if (count(16, wr = 32) <= kTiles || count(16, wr = 64) <= kTiles) return;
+  if (M > 16) {
+    tile = 32;
+    if (count(32, wr = 64) <= kTiles) return;
+  }
+  wr = 128;
+  if (M > 32 && count(32, 128) > kTiles) tile = 64;
+}
+
+// Grouped: `tile` rows of A at a time, which belong to one expert; M a multiple of it.
 template <bool FP8>
 static int run(const void* a, const void* w, Params p, int n_experts, int tile, int K, int64_t lda, int64_t ldw, cudaStream_t s) {
   constexpr int KE = FP8 ? 128 : 64;
+  int wr = 128;
+  if (FP8 && p.tile_expert == nullptr) fp8_tile(p.M, p.N, tile, wr);
   if ((tile != 16 && tile != 32 && tile != 64) || n_experts < 1 || (p.tile_expert != nullptr && (p.M % tile || p.N % 128)) ||
       (((uintptr_t)a | (uintptr_t)w | (uintptr_t)p.c) & 15))
     return (int)cudaErrorInvalidValue;
   p.k_blocks = (K + KE - 1) / KE;
   p.x_rows = p.M >= tile ? tile : ((p.M + 7) & ~7);
-  const int64_t tiles = (int64_t)((p.M + tile - 1) / tile) * ((p.N + 127) / 128);
+  const int64_t tiles = (int64_t)((p.M + tile - 1) / tile) * ((p.N + wr - 1) / wr);
   if (tiles > 65535) return (int)cudaErrorInvalidValue;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -366,10 +442,15 @@ static int run(const void* a, const void* w, Params p, int n_experts, int tile, 
   }
   p.err = g_err[dev & 63];
   // a grouped launch holds tiles of experts nobody chose: how many are live is not known here, and there are many
-  const int splits = p.tile_expert != nullptr ? 1 : choose_split((int)tiles, p.k_blocks);
-  if (tile == 16) return launch<16, FP8>(a, w, p, K, lda, ldw, n_experts, splits, dev, s);
-  if (tile == 32) return launch<32, FP8>(a, w, p, K, lda, ldw, n_experts, splits, dev, s);
-  return launch<64, FP8>(a, w, p, K, lda, ldw, n_experts, splits, dev, s);
+  const int splits = FP8 || p.tile_expert != nullptr ? 1 : choose_split((int)tiles, p.k_blocks);
+  const auto go = [&](auto kernel) { return kernel(a, w, p, K, lda, ldw, n_experts, splits, dev, s); };
+  if constexpr (FP8) {
+    if (wr == 32) return go(launch<16, true, 32, 4>);
+    if (wr == 64) return go(tile == 16 ? launch<16, true, 64, 2> : launch<32, true, 64, 2>);
+    return go(tile == 16 ? launch<16, true, 128, 2> : (tile == 32 ? launch<32, true, 128, 2> : launch<64, true, 128, 2>));
+  } else {
+    return go(tile == 16 ? launch<16, false, 128, 1> : (tile == 32 ? launch<32, false, 128, 1> : launch<64, false, 128, 1>));
+  }
 }
 
 static Params make_params(void* c, int64_t ldc, int M, int N, const void* tile_expert) {
@@ -415,14 +496,14 @@ XLLM_API int xllm_gemm_bf16_grouped_few(const void* a, const void* w, void* c, c
   return run<false>(a, w, p, n_experts, tile, K, lda, K, (cudaStream_t)stream);
 }
 
-// The contracts of xllm_gemm_fp8_block and (tile_expert not null) xllm_gemm_fp8_block_grouped, `tile` rows of A (16, 32 or 64)
-// at a time.
+// The contracts of xllm_gemm_fp8_block, for up to 64 rows, and (tile_expert not null) xllm_gemm_fp8_block_grouped, `tile` rows of A
+// (16, 32 or 64) at a time, with the same sums in the same order.  K of at most 49152.
 XLLM_API int xllm_gemm_fp8_few(const void* a, const void* w, void* c, const void* a_scale, const void* w_scale,
                                const void* tile_expert, int n_experts, int tile, int M, int N, int K, int64_t lda, int64_t ldw,
                                int64_t ldc, void* stream) {
   using namespace xllm::few;
   if (M == 0 || N == 0) return 0;
-  if (K % 128 || K <= 0 || N % 8 || lda % 16 || ldw % 16) return (int)cudaErrorInvalidValue;
+  if (K % 128 || K <= 0 || K > kFp8MaxK || N % 8 || lda % 16 || ldw % 16 || (tile_expert == nullptr && M > 64)) return (int)cudaErrorInvalidValue;
   Params p = make_params(c, ldc, M, N, tile_expert);
   p.a_scale = (const float*)a_scale; p.w_scale = (const float*)w_scale;
   return run<true>(a, w, p, n_experts, tile, K, lda, ldw, (cudaStream_t)stream);

@@ -23,7 +23,8 @@ _lib.register_signature("xllm_gemm_fp8_few", [P, P, P, P, P, P, I, I, I, I, I, L
 _lib.register_signature("xllm_act_quant_fp8_group128", [P, P, P, L, I, P, I, I, F, F, P])
 
 FP8 = torch.float8_e4m3fn
-FEW_ROWS = 64        # most rows of the product whose tile is 128 weight rows (csrc/kernels/gemm_few.cu)
+FEW_ROWS = 64        # most rows of the product whose tile has weights for rows (csrc/kernels/gemm_few.cu), and its longest K:
+FEW_K = 49152        # the scales of a tile lie in shared memory
 FP8_MAX = 448.0
 
 
@@ -164,10 +165,9 @@ def block_scaled_mm(a_q, a_scale, w_q, w_scale, out=None):
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=a_q.device)
     # few rows: bound by the weights' way from HBM; from 65 rows on a tile of 128 rows of a_q wastes less than two passes
-    if 0 < M <= FEW_ROWS:
-        check(_lib.load().xllm_gemm_fp8_few(ptr(a_q), ptr(w_q), ptr(out), ptr(a_scale), ptr(w_scale), None, 1,
-                                            16 if M <= 16 else 32 if M <= 32 else 64, M, N, K, a_q.stride(0), w_q.stride(0),
-                                            out.stride(0), stream()), "gemm_fp8_few")
+    if 0 < M <= FEW_ROWS and K <= FEW_K:
+        check(_lib.load().xllm_gemm_fp8_few(ptr(a_q), ptr(w_q), ptr(out), ptr(a_scale), ptr(w_scale), None, 1, 0, M, N, K,
+                                            a_q.stride(0), w_q.stride(0), out.stride(0), stream()), "gemm_fp8_few")
         from . import _count
         _count()
         return out

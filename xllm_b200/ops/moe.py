@@ -13,6 +13,7 @@ import torch
 
 from . import _lib, glu
 from ._lib import F, I, L, P, check, ptr, stream
+from .fp8 import FEW_K
 
 _lib.register_signature("xllm_moe_route", [P, I, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P])
 _lib.register_signature("xllm_moe_route_ld", [P, L, I, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P])
@@ -168,6 +169,8 @@ def fused_moe(x, logits, w_gate_up, w_down, top_k, scoring="softmax", bias=None,
     simt = w_scales is None and (dt == 1 or H % 8 or I2 % 64 or inter % 8 or Y % 64)
     tile = 128 if simt or I2 % 128 or Y % 128 else row_tile(T, top_k, E)
     if tile == 256 and (w_scales is not None or I2 % 256 or Y % 256):
+        tile = 128
+    if w_scales is not None and max(H, inter) > FEW_K:
         tile = 128
     # rows that T tokens can take: a workspace is made for more
     rows = min(ws.rows, (T * top_k + min(E_local, T * top_k) * (tile - 1) + tile - 1) // tile * tile)
