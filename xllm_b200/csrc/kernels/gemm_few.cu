@@ -137,7 +137,6 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
     __syncwarp();
   }
   pdl_wait();
-  pdl_launch_dependents();
   int expert = 0;
   if (p.tile_expert != nullptr) {
     expert = p.tile_expert[mt];
@@ -150,6 +149,9 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // Not before the allocation: a dependent block that came first could take this SM's tensor memory and keep it in its own wait
+  // for this grid, which would then wait for it without end.
+  pdl_launch_dependents();
   const uint32_t tmem = *tmem_holder;
   const int m0 = mt * TN, n0 = nt * WR;
   const int live = min(TN, p.M - m0);
