@@ -159,9 +159,9 @@ __global__ void __launch_bounds__(256, RUN > 1 ? 3 : 2) gdn_conv_kernel(GdnParam
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       s[j] = x0[0][j] * w[0][j];
-      if (back >= 1) s[j] += x0[1][j] * w[1][j];
-      if (back >= 2) s[j] += x0[2][j] * w[2][j];
-      if (back >= 3) s[j] += x0[3][j] * w[3][j];
+#pragma unroll
+      for (int t = 1; t <= K1; ++t)
+        if (back >= t) s[j] += x0[t][j] * w[t][j];
     }
     bf16* tail = p.tail + ((int64_t)slot * C + ch) * K1;            // [channel][input], oldest first
     if (back < K1 && on) {
@@ -173,9 +173,10 @@ __global__ void __launch_bounds__(256, RUN > 1 ? 3 : 2) gdn_conv_kernel(GdnParam
 #pragma unroll
       for (int u = 0; u < K1; ++u) {                                // u + 1 inputs before the sequence's rows
         const int t = u + 1 + back;
+        if (t > K1) break;                                          // (zero times what is not finite would not be zero)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          s[j] += __bfloat162float(past[j * K1 + K1 - 1 - u]) * (t == 1 ? w[1][j] : (t == 2 ? w[2][j] : (t == 3 ? w[3][j] : 0.f)));
+          s[j] += __bfloat162float(past[j * K1 + K1 - 1 - u]) * (t == 1 ? w[1][j] : (t == 2 ? w[2][j] : w[3][j]));
       }
       if (n == 1) {                                                 // this lane alone reads these inputs: move them up
         __align__(8) bf16 now[4 * K1];
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(256, 2) gdn_step_kernel(GdnParams p) {
 //
 // Every decay is at most 1.  y and v are bf16 as the convolution leaves them, so that their products on the tensor cores are
 // exact and accumulate in fp32; S, U, M and P are fp32 values as three bf16 terms (24 bits), of which products below 2^-24 of
-// the largest are left out.  gdn_prep_kernel makes M, P and the factors, all chunks side by side; gdn_chunk_kernel walks the
+// the largest are left out.  (A chunk with anything that is not finite goes token by token.)  gdn_prep_kernel makes M, P and the factors, all chunks side by side; gdn_chunk_kernel walks the
 // chunks of a sequence: a warp owns 16 state columns for all of dk as accumulators of S^T, which are the A operand of S^T Y^T
 // without leaving the registers, as U^T is of the products behind it.
 //
@@ -376,7 +377,9 @@ __global__ void __launch_bounds__(128) gdn_prep_kernel(GdnParams p) {
       const double x = __shfl_up_sync(0xffffffffu, G, o);
       if (lane >= o) G += x;
     }
-    const double end = __shfl_sync(0xffffffffu, G, kGC - 1);
+    // a decay to zero within one token, or NaN: differences of its sums say nothing, and no token is a NaN end
+    const bool finite = __all_sync(0xffffffffu, fabs(G) < (double)INFINITY);
+    const double end = finite ? __shfl_sync(0xffffffffu, G, kGC - 1) : (double)NAN;
     if (lane < kGC) {
       gs[warp][lane] = G;
       const float e = expf((float)G);
@@ -407,9 +410,48 @@ __global__ void __launch_bounds__(128) gdn_prep_kernel(GdnParams p) {
   }
 }
 
+// n tokens from row0 on one after the other, for 16 columns of a state that lies in memory as the accumulators of the walk below
+// (what a lane reads of it is what the lane wrote).  For chunks with anything that is not finite: by the chunk, zeros of M and P
+// would carry it to tokens in front of it, and an infinite state has no three terms.
+template <int DK>
+__device__ __noinline__ void gdn_walk_tokens(const GdnParams& p, float* S, int row0, int n, int h, int g, int vrow, int kc) {
+  const int dk = p.dk, dv = p.dv;
+  for (int64_t row = row0; row < row0 + n; ++row) {
+    const float2 gb = p.gb[row * p.H + h];
+    const float decay = expf(gb.x), fk = p.fk[row * p.G + g], fq = p.fq[row * p.G + g];
+    const bf16 *yk = p.yk + (row * p.G + g) * DK, *yq = p.yq + (row * p.G + g) * DK, *yv = p.yv + (row * p.H + h) * p.dvp;
+    float d[2] = {0.f, 0.f}, o[2] = {0.f, 0.f};
+    for (int i = 0; i < DK / 4; ++i) {
+      const int c = (i >> 1) * 8 + kc + (i & 1);
+      for (int u = 0; u < 2; ++u)
+        if (c < dk && vrow + 8 * u < dv) d[u] += S[(int64_t)c * dv + vrow + 8 * u] * decay * (__bfloat162float(yk[c]) * fk);
+    }
+    for (int u = 0; u < 2; ++u) {
+      d[u] += __shfl_xor_sync(0xffffffffu, d[u], 1);
+      d[u] += __shfl_xor_sync(0xffffffffu, d[u], 2);
+      if (vrow + 8 * u < dv) d[u] = gb.y * (__bfloat162float(yv[vrow + 8 * u]) - d[u]);
+    }
+    for (int i = 0; i < DK / 4; ++i) {
+      const int c = (i >> 1) * 8 + kc + (i & 1);
+      for (int u = 0; u < 2; ++u)
+        if (c < dk && vrow + 8 * u < dv) {
+          float* at = S + (int64_t)c * dv + vrow + 8 * u;
+          const float x = *at * decay + __bfloat162float(yk[c]) * fk * d[u];
+          *at = x;
+          o[u] += x * (__bfloat162float(yq[c]) * fq);
+        }
+    }
+    for (int u = 0; u < 2; ++u) {
+      o[u] += __shfl_xor_sync(0xffffffffu, o[u], 1);
+      o[u] += __shfl_xor_sync(0xffffffffu, o[u], 2);
+      if (kc == 0 && vrow + 8 * u < dv) p.o[(row * p.H + h) * dv + vrow + 8 * u] = o[u];
+    }
+  }
+}
+
 // grid (slices of 64 columns, heads, prompts)
 template <int DK>
-__global__ void __launch_bounds__(32 * kGWarps, 2) gdn_chunk_kernel(GdnParams p) {
+__global__ void __launch_bounds__(32 * kGWarps, 2) gdn_chunk_kernel(const __grid_constant__ GdnParams p) {
   constexpr int CH = DK / 8, NT = 32 * kGWarps, TILE = kGC * DK * 2;
   constexpr int V_OFF = 2 * TILE, B_OFF = V_OFF + kGC * kGVld * 2, STAGE = (B_OFF + GdnBlob::bytes + 127) / 128 * 128;
   static_assert(kGStages * STAGE <= 48 * 1024, "static limit of dynamic shared memory");
@@ -518,13 +560,18 @@ __global__ void __launch_bounds__(32 * kGWarps, 2) gdn_chunk_kernel(GdnParams p)
 #pragma unroll
       for (int e = 0; e < 2; ++e) f[i][e] = fs[8 * i + kc + e];
     uint32_t xh[4], xm[4], xl[4];
+    // every term of bf16: an infinite state, or input, is seen in the products with it, whatever they are multiplied with
+    bool tame = fabsf(f[0][0].w) <= 1.f;
+    const auto is_tame = [](float x) { return fabsf(x) < 3.38e38f; };
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const bf16* v = vs + (8 * i + kc) * kGVld + vloc + 8 * u;
-        split3(__bfloat162float(v[0]) - f[i][0].x * (w[i][2 * u] + wl[i][2 * u]),
-               __bfloat162float(v[kGVld]) - f[i][1].x * (w[i][2 * u + 1] + wl[i][2 * u + 1]), xh[2 * i + u], xm[2 * i + u], xl[2 * i + u]);
+        const float x = __bfloat162float(v[0]) - f[i][0].x * (w[i][2 * u] + wl[i][2 * u]);
+        const float y = __bfloat162float(v[kGVld]) - f[i][1].x * (w[i][2 * u + 1] + wl[i][2 * u + 1]);
+        tame = tame && is_tame(x) && is_tame(y);
+        split3(x, y, xh[2 * i + u], xm[2 * i + u], xl[2 * i + u]);
       }
     const uint32_t small = st + B_OFF + (uint32_t)(brow * kGC * 2 + bcb * 16);
     float uu[2][4], pu[2][4];
@@ -547,6 +594,25 @@ __global__ void __launch_bounds__(32 * kGWarps, 2) gdn_chunk_kernel(GdnParams p)
       }
     };
     product(uu, GdnBlob::m);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) tame = tame && is_tame(uu[i][e]);
+    if (!__all_sync(0xffffffffu, tame)) {
+      const auto elements = [&](auto&& f) {
+#pragma unroll
+        for (int nt = 0; nt < DK / 8; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int c = nt * 8 + kc + (e & 1), v = vrow + (e >> 1) * 8;
+            if (c < dk && v < dv) f(acc[nt][e], S[(int64_t)c * dv + v]);
+          }
+      };
+      elements([](float a, float& m) { m = a; });
+      gdn_walk_tokens<DK>(p, S, row0 + j * kGC, n, h, g, vrow, kc);
+      elements([](float& a, float m) { a = m; });
+      continue;
+    }
     // ---- O^T
 #pragma unroll
     for (int i = 0; i < 2; ++i)
