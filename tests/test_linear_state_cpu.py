@@ -6,6 +6,7 @@ import torch
 from xllm_b200 import LLM, SamplingParams
 from xllm_b200.engine.llm_engine import EngineConfig, LLMEngine
 from xllm_b200.models import ModelArgs
+from xllm_b200.models.qwen3_next import GatedDeltaNet
 
 
 def _args():
@@ -36,3 +37,22 @@ def test_preemption_and_chunking_do_not_change_the_stream():
     assert got == want
     assert tight.engine.scheduler.num_preemptions > 0
     assert not tight.engine.model.state.owner and len(tight.engine.model.state.free) == 7
+
+
+def test_layers_of_tensor_operations_ask_the_device_nothing(monkeypatch):
+    """Where a layer runs on tensor operations, begins and lengths of sequences come from the lists that the engine has on the host:
+    read off the device they would stop every layer until it has caught up."""
+    llm, seen = _make(num_blocks=32, max_tokens_per_batch=64), []
+    forward = GatedDeltaNet.forward
+
+    def without(self, x, meta, state):
+        seen.append(len(meta.seq_bounds))
+        on_device, meta.cu_q, meta.kv_lens = (meta.cu_q, meta.kv_lens), None, None
+        y = forward(self, x, meta, state)
+        meta.cu_q, meta.kv_lens = on_device
+        return y
+
+    monkeypatch.setattr(GatedDeltaNet, "__call__", without)
+    assert not llm.engine.model.state_on_device and not llm.engine.model.supports_graph
+    out = llm.generate([[5, 6, 7], [9]], SamplingParams(max_tokens=3, temperature=0.0, ignore_eos=True))
+    assert all(len(o.outputs[0].token_ids) == 3 for o in out) and max(seen) == 2

@@ -110,9 +110,7 @@ class GatedDeltaNet(Module):
         beta = torch.sigmoid(b.reshape(T, nv).float())
         g = -self.A_log.float().exp() * F.softplus(a.reshape(T, nv).float() + self.dt_bias.float())
         conv, rec = state.conv[self.lin_idx], state.rec[self.lin_idx]
-        cu, lens, slots = meta.cu_q.tolist(), meta.kv_lens.tolist(), meta.state_slots.long()
-        bounds = list(zip(cu[:-1], cu[1:]))
-        fresh = [n == e - b for (b, e), n in zip(bounds, lens)]
+        slots, fresh, bounds = meta.state_slots, meta.state_fresh, meta.seq_bounds
         out = torch.empty(T, nv, dv, dtype=torch.float32, device=x.device)
 
         def heads(y):                                      # conv output rows -> normalised, scaled q / k and v per value head
@@ -214,7 +212,6 @@ class NextDecoderLayer(DecoderLayer):
 class Qwen3NextCausalLM(DenseCausalLM):
     fused_tp = False
     needs_state = True
-    state_on_device = True          # state slots are a device input of the step: graphs capture it
 
     def __init__(self, args, dtype=torch.bfloat16, device="cpu", ps=None):
         e = dict(args.extra)
@@ -240,8 +237,12 @@ class Qwen3NextCausalLM(DenseCausalLM):
         self.state = None
 
     @property
-    def supports_graph(self):
+    def state_on_device(self):
+        """Whether the state slots are a device input of the step, so that graphs capture it.  Layers that run on tensor
+        operations take them, and where sequences begin and which start afresh, from the host."""
         return all(l.mixer.fused is not None for l in self.layers if l.linear)
+
+    supports_graph = state_on_device
 
     @property
     def num_kv_heads_local(self):
