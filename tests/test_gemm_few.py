@@ -152,3 +152,31 @@ def test_expert_layer(T, E, K, fp8_weights):
     # bf16: three roundings.  fp8: three factors of an output (gate, up through x; the activation) carry a rounding to e4m3 each,
     # uniform within 2^-4 of a value at worst, that is 2^-4 / sqrt(3) in the mean square, and independent: 2^-4 together
     _close(got, want, 2 ** -4 if scales else 2 ** -7)
+
+
+_CAPTURE_FIRST = """
+import torch
+from xllm_b200.ops import fp8, gemm_tcgen05
+x, w = (torch.randn(n, 256, device="cuda").bfloat16() for n in (96, 512))
+a, a_s = fp8.quant_group128(x)
+b, b_s = fp8.quant_block128_ref(w.float())
+gemm_tcgen05.prepare()
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    got = [gemm_tcgen05.gemm_nt(x[:4], w), fp8.block_scaled_mm(a[:4], a_s[:4], b, b_s), gemm_tcgen05.gemm_nt(x, w)]
+graph.replay()
+want = x.double() @ w.double().T
+for y, n, rel in zip(got, (4, 4, 96), (2 ** -8, 2 ** -3, 2 ** -8)):
+    assert (y.double() - want[:n]).norm() <= rel * want[:n].norm()
+assert gemm_tcgen05.error_status() == 0
+print("captured")
+"""
+
+
+def test_the_first_launches_may_be_captured():
+    """prepare() leaves nothing to allocate: a process captures its first products."""
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", _CAPTURE_FIRST], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]

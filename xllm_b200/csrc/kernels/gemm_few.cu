@@ -29,6 +29,7 @@
 // (xllm_gemm_few_error_status).
 #include "tc_common.cuh"
 #include <atomic>
+#include <mutex>
 
 namespace xllm {
 namespace few {
@@ -340,7 +341,20 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant
   }
 }
 
-static int* g_err[64] = {};
+static std::atomic<int*> g_err[64] = {};
+
+// The error word of a device, made at its first launch or by xllm_gemm_few_prepare (a capture allows no allocation), or null.
+static int* error_word(int dev) {
+  static std::mutex making;
+  int* word = g_err[dev & 63].load(std::memory_order_acquire);
+  if (word != nullptr) return word;
+  const std::lock_guard<std::mutex> lock(making);
+  word = g_err[dev & 63].load(std::memory_order_acquire);
+  if (word != nullptr) return word;
+  if (cudaMalloc(&word, sizeof(int)) != cudaSuccess || cudaMemset(word, 0, sizeof(int)) != cudaSuccess) return nullptr;
+  g_err[dev & 63].store(word, std::memory_order_release);
+  return word;
+}
 
 // [rows, cols] with row stride ld elements; box = [box_rows, 128 bytes], 128-byte swizzle
 static bool make_map_of(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows, bool fp8) {
@@ -438,11 +452,8 @@ static int run(const void* a, const void* w, Params p, int n_experts, int tile, 
   if (tiles > 65535) return (int)cudaErrorInvalidValue;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (g_err[dev & 63] == nullptr) {
-    if (cudaMalloc(&g_err[dev & 63], sizeof(int)) != cudaSuccess) return (int)cudaErrorMemoryAllocation;
-    cudaMemset(g_err[dev & 63], 0, sizeof(int));
-  }
-  p.err = g_err[dev & 63];
+  p.err = error_word(dev);
+  if (p.err == nullptr) return (int)cudaErrorMemoryAllocation;
   // a grouped launch holds tiles of experts nobody chose: how many are live is not known here, and there are many
   const int splits = FP8 || p.tile_expert != nullptr ? 1 : choose_split((int)tiles, p.k_blocks);
   const auto go = [&](auto kernel) { return kernel(a, w, p, K, lda, ldw, n_experts, splits, dev, s); };
@@ -511,14 +522,21 @@ XLLM_API int xllm_gemm_fp8_few(const void* a, const void* w, void* c, const void
   return run<true>(a, w, p, n_experts, tile, K, lda, ldw, (cudaStream_t)stream);
 }
 
-// 0 = no bounded wait expired in these kernels on this device since the last call.
-XLLM_API int xllm_gemm_few_error_status() {
-  using namespace xllm::few;
+// What launches on this device need, ahead of a capture.
+XLLM_API int xllm_gemm_few_prepare() {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (g_err[dev & 63] == nullptr) return 0;
+  return xllm::few::error_word(dev) != nullptr ? 0 : (int)cudaErrorMemoryAllocation;
+}
+
+// 0 = no bounded wait expired in these kernels on this device since the last call.
+XLLM_API int xllm_gemm_few_error_status() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int* word = xllm::few::g_err[dev & 63].load(std::memory_order_acquire);
+  if (word == nullptr) return 0;
   int v = 0;
-  cudaMemcpy(&v, g_err[dev & 63], sizeof(int), cudaMemcpyDeviceToHost);
-  if (v != 0) cudaMemset(g_err[dev & 63], 0, sizeof(int));
+  cudaMemcpy(&v, word, sizeof(int), cudaMemcpyDeviceToHost);
+  if (v != 0) cudaMemset(word, 0, sizeof(int));
   return v;
 }

@@ -1764,6 +1764,10 @@ XLLM_API int xllm_gemm_prepare() {
   using namespace xllm;
   int dev = 0;
   cudaGetDevice(&dev);
+  if (g_err_word[dev & 63] == nullptr) {
+    if (cudaMalloc(&g_err_word[dev & 63], sizeof(int)) != cudaSuccess) return (int)cudaErrorMemoryAllocation;
+    cudaMemset(g_err_word[dev & 63], 0, sizeof(int));
+  }
   return split_scratch_ready(dev, nullptr) ? 0 : (int)cudaErrorMemoryAllocation;
 }
 

@@ -13,6 +13,7 @@ _lib.register_signature("xllm_gemm_bf16", [P, P, P, P, I, I, I, L, L, L, I, I, I
 _lib.register_signature("xllm_gemm_error_status", [], I)
 _lib.register_signature("xllm_gemm_few_error_status", [], I)
 _lib.register_signature("xllm_gemm_prepare", [], I)
+_lib.register_signature("xllm_gemm_few_prepare", [], I)
 _lib.register_signature("xllm_gemm_set_k_per_stage", [I], None)
 _lib.register_signature("xllm_gemm_set_dual_issue", [I], None)
 _lib.register_signature("xllm_pack_weight_bf16", [P, P, I, I, L, P])
@@ -171,8 +172,9 @@ def set_dual_issue(on: bool):
 
 
 def prepare():
-    """Allocate the split-K scratch of the current device (before CUDA-graph capture)."""
+    """Allocate the split-K scratch and the error words of the current device (before CUDA-graph capture)."""
     check(_lib.load().xllm_gemm_prepare(), "gemm_prepare")
+    check(_lib.load().xllm_gemm_few_prepare(), "gemm_few_prepare")
 
 
 def error_status() -> int:
