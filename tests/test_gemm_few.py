@@ -120,6 +120,32 @@ def test_grouped(tile, kind):
         _close(got, want, 2 ** -7 if kind == "gated" else 2 ** -8)
 
 
+@pytest.mark.parametrize("kind", ["bf16", "fp8"])
+def test_grouped_with_more_tiles_than_a_grid_has_rows(kind):
+    """65664 of them, as hundreds of experts with wide rows have; a grid's second and third size end at 65535."""
+    from xllm_b200.ops import _lib
+    from xllm_b200.ops._lib import check, ptr, stream
+    g = torch.Generator(device=DEV).manual_seed(5)
+    M, N, K, tile, E = 513 * 16, 128 * 128, 128, 16, 2
+    x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(E, N, K, device=DEV, generator=g) * K ** -0.5).bfloat16()
+    experts = (torch.arange(M // tile, device=DEV) % E).int()
+    out = torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    if kind == "fp8":
+        a, a_s = fp8.quant_group128(x)
+        parts = [fp8.quant_block128_ref(w[e].float()) for e in range(E)]
+        fp8.block_scaled_mm_grouped(a, a_s, torch.stack([p[0] for p in parts]), torch.stack([p[1] for p in parts]), experts, out, tile)
+        x = a.float() * a_s.repeat_interleave(128, 1)
+        w = torch.stack([fp8.dequant_block128_ref(q, s, torch.float32) for q, s in parts])
+    else:
+        check(_lib.load().xllm_gemm_bf16_grouped_few(ptr(x), ptr(w), ptr(out), ptr(experts), tile, M, N, K, E, K, N, 0, 0.0, 0.0,
+                                                     stream()), "few")
+    rows = torch.arange(M, device=DEV).view(-1, tile)
+    for e in range(E):
+        here = rows[experts == e].flatten()
+        _close(out[here], x[here].double() @ w[e].double().T, 2 ** -8)
+
+
 @pytest.mark.parametrize("rows,d,act", [(1, 128, "silu"), (48, 2048, "silu"), (33, 384, "gelu_tanh")])
 def test_activation_and_its_quantisation(rows, d, act):
     from xllm_b200 import ops
