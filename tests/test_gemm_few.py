@@ -120,6 +120,39 @@ def test_grouped(tile, kind):
         _close(got, want, 2 ** -7 if kind == "gated" else 2 ** -8)
 
 
+@pytest.mark.parametrize("experts", [[1, 1, 1, 1, 0, 0, 0, 0], [0, -1, 1, 1, 0, 1, 0] + [-1] * 40, [-1] * 9])
+@pytest.mark.parametrize("N,K", [(8192, 5120), (512, 4352)])
+@pytest.mark.parametrize("kind", ["bf16", "pair", "fp8"])
+def test_grouped_tile_orders(kind, N, K, experts):
+    """Experts above what the L2 keeps, whose column tiles are swept by all row tiles, and small ones; tiles that nobody has among the
+    others, behind them, and alone."""
+    from xllm_b200.ops import _lib
+    from xllm_b200.ops._lib import check, ptr, stream
+    g = torch.Generator(device=DEV).manual_seed(N)
+    E, tile = 2, 256 if kind == "pair" else 128
+    experts = torch.tensor(experts, dtype=torch.int32, device=DEV)
+    M = len(experts) * tile
+    x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(E, N, K, device=DEV, generator=g) * K ** -0.5).bfloat16()
+    out = torch.full((M, N), 7.0, device=DEV, dtype=torch.bfloat16)
+    if kind == "fp8":
+        a, a_s = fp8.quant_group128(x)
+        parts = [fp8.quant_block128_ref(w[e].float()) for e in range(E)]
+        fp8.block_scaled_mm_grouped(a, a_s, torch.stack([p[0] for p in parts]), torch.stack([p[1] for p in parts]), experts, out)
+        x = a.float() * a_s.repeat_interleave(128, 1)
+        w = torch.stack([fp8.dequant_block128_ref(q, s, torch.float32) for q, s in parts])
+    elif kind == "pair":
+        check(_lib.load().xllm_gemm_bf16_grouped_pair(ptr(x), ptr(w), ptr(out), ptr(experts), M, N, K, E, K, N, 0, 0.0, 0.0, stream()), "pair")
+    else:
+        check(_lib.load().xllm_gemm_bf16_grouped(ptr(x), ptr(w), ptr(out), ptr(experts), M, N, K, E, K, N, stream()), "grouped")
+    for i, e in enumerate(experts.tolist()):
+        got = out[i * tile:(i + 1) * tile]
+        if e < 0:
+            assert (got == 7).all()
+        else:
+            _close(got, x[i * tile:(i + 1) * tile].double() @ w[e].double().T, 2 ** -8)
+
+
 @pytest.mark.parametrize("kind", ["bf16", "fp8"])
 def test_grouped_with_more_tiles_than_a_grid_has_rows(kind):
     """65664 of them, as hundreds of experts with wide rows have; a grid's second and third size end at 65535."""

@@ -146,6 +146,7 @@ struct GemmMode {
   // group, into an output of N / 2 columns.  0 = off, 1 = SiLU, 2 = GELU(erf), 3 = GELU(tanh), 4 = clamped_glu.
   int act_mul;
   float act_limit, act_alpha;
+  int sweep;               // grouped: the row tiles of a column tile are neighbours (sweep_rows())
 };
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
@@ -524,20 +525,19 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   volatile int* s_last = reinterpret_cast<volatile int*>(tmem_holder + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tiles = (M + kBM - 1) / kBM, n_tiles = (N + BN - 1) / BN;
-  const int total_tiles = m_tiles * n_tiles;
-  // Row tiles are neighbours, so that CTAs at work together share a tile's weights; grouped by expert, the column tiles of a row
-  // tile are: the experts' weights are read once either way, but all experts' rows (prompts: more than the L2 holds beside
-  // them) would be read again for every column tile (25 thousand rows of 2048 for 128 experts, one B200: 230 us, now 181 us
-  // with 1536 columns, 180 us, now 125 us for the product back).
-  const auto tile_m = [&](int t) { return tile_expert != nullptr ? t / n_tiles : t % m_tiles; };
-  const auto tile_n = [&](int t) { return tile_expert != nullptr ? t % n_tiles : t / m_tiles; };
+  const int n_tiles = (N + BN - 1) / BN;
+  int m_tiles = (M + kBM - 1) / kBM, total_tiles = m_tiles * n_tiles;
+  // Row tiles are neighbours, so that CTAs at work together share a tile's weights; grouped by expert, mostly the column tiles of a
+  // row tile are (sweep_rows())
+  const bool across = tile_expert != nullptr && !mode.sweep;
+  const auto tile_m = [&](int t) { return across ? t / n_tiles : t % m_tiles; };
+  const auto tile_n = [&](int t) { return across ? t % n_tiles : t / m_tiles; };
   const int k_elems = mode.fp8 ? 2 * kBK : kBK;  // elements per 128-byte K block
   const int k_blocks = (K + k_elems - 1) / k_elems;
   const int ks = mode.ks;
   const int k_steps = (k_blocks + KS - 1) / KS;  // ring stages along K (a tail block past K reads as zeros)
   const int kbs = (k_steps + ks - 1) / ks;       // stages per split
-  const int total_units = total_tiles * ks;
+  int total_units = total_tiles * ks;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -562,6 +562,18 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   const uint32_t tmem_base = *tmem_holder;
   pdl_wait();
   pdl_launch_dependents();  // dependents may be scheduled now; they block in their own pdl_wait()
+  if (mode.sweep) {        // tiles that nobody has lie behind the others: among them, CTAs would get unequal shares
+    while (m_tiles > 0) {
+      const int i = m_tiles - 1 - lane;
+      const uint32_t used = __ballot_sync(0xffffffffu, i >= 0 && tile_expert[max(i, 0)] >= 0);
+      if (used != 0) {
+        m_tiles -= __ffs(used) - 1;
+        break;
+      }
+      m_tiles = max(m_tiles - 32, 0);
+    }
+    total_units = total_tiles = m_tiles * n_tiles;
+  }
 
   if (warp == 0) {
     {
@@ -850,7 +862,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const _
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int m_tiles = (M + 2 * kBM - 1) / (2 * kBM), n_tiles = (N + BN - 1) / BN;
   const int total_tiles = m_tiles * n_tiles;
-  // grouped by expert (see gemm_bf16_tcgen05_kernel): a row tile of 256 belongs to one, expert e's weights are rows e N ..
+  // grouped by expert (sweep_rows()): a row tile of 256 belongs to one, expert e's weights are rows e N ..
   const auto tile_m = [&](int t) { return tile_expert != nullptr ? t / n_tiles : t % m_tiles; };
   const auto tile_n = [&](int t) { return tile_expert != nullptr ? t % n_tiles : t / m_tiles; };
   const auto expert_of = [&](int t) { return tile_expert != nullptr ? tile_expert[tile_m(t)] : 0; };
@@ -1124,6 +1136,22 @@ static int usable_split(int ks, int M, int N, int K, int k_per_stage, int counte
   return ks;
 }
 
+// Order of a grouped product's tiles in rows of 128, sorted by expert: the column tiles of a row tile side by side read the rows once
+// and an expert's weights for every row tile, from L2 if they stay there or while all of the expert's tiles are at work together;
+// the row tiles of a column tile side by side read the weights once and the rows for every column tile.  So the second where an
+// expert's weights are more than half the L2 and its tiles more than most SMs, unless the rows are far more than the L2.
+// Measured (one B200, us, first and second; experts x N x K, row tiles an expert):
+//   8 x 28672 x 4096    1: 341, 343    2: 570, 456    3: 838, 636    6: 1640, 1211    20: 5100, 4433
+//   16 x 16384 x 5120   1: 438, 460    3: 1118, 949   8: 3000, 2566       8 x 8192 x 5120    2: 181, 177    4: 298, 278
+//   64 x 12288 x 4096   1: 1056, 1260  3: 2707, 2745                      8 x 4096 x 14336   6: 644, 639    12: 1190, 1273
+//   128 x 1536 x 2048   2: 216, 282                                       128 x 2048 x 768   2: 120, 149
+// Row tiles of 256 (CTA pairs) gain in two of eighteen such sizes, by 6 %, and lose up to a third; block-scaled e4m3 in none.
+static bool sweep_rows(int M, int N, int K, int bn, int n_experts) {
+  const double weights = 2. * N * K, rows = 2. * M * K;
+  const double tiles = ((double)M / kBM / n_experts - 0.5) * N / bn;        // of an expert; half a row tile is padding
+  return weights > 64e6 && rows < 256e6 && tiles > 111;
+}
+
 template <int BN, int STAGES, int KS = 1, bool DUAL = false>
 static int launch_gemm(const void* a, const void* w, void* c, const void* bias, int M, int N, int K, int64_t lda,
                        int64_t ldw, int64_t ldc, int max_ctas, int w_packed, cudaStream_t s,
@@ -1153,6 +1181,7 @@ static int launch_gemm(const void* a, const void* w, void* c, const void* bias, 
   // gated-activation epilogue: the output has one column per (gate, up) pair, half of the GEMM's N
   else if (!make_tmap(&tc, c, M, mode.act_mul ? N / 2 : N, ldc, 32, false)) return (int)cudaErrorInvalidValue;
   const int tiles = ((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
+  mode.sweep = tile_expert != nullptr && sweep_rows(M, N, K, BN, n_experts);
   if (split_k > 1 && tile_expert == nullptr && !mode.fp8) {
     mode.ks = usable_split(split_k, M, N, K, KS, tiles, dev, s);
     mode.ws = g_split_ws[dev & 63];
@@ -1280,7 +1309,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (M + kBM - 1) / kBM, n_tiles = (N + BN - 1) / BN;
   const int total_tiles = m_tiles * n_tiles;
-  const auto tile_m = [&](int t) { return tile_expert != nullptr ? t / n_tiles : t % m_tiles; };   // as in gemm_bf16_tcgen05_kernel
+  const auto tile_m = [&](int t) { return tile_expert != nullptr ? t / n_tiles : t % m_tiles; };   // see sweep_rows()
   const auto tile_n = [&](int t) { return tile_expert != nullptr ? t % n_tiles : t / m_tiles; };
   const int k_blocks = K / 128;
 
