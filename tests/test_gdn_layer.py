@@ -231,21 +231,40 @@ def test_sigmoid_gate(T, heads, d):
     assert ((got - want).abs() <= 2 ** -7 * want.abs() + 1e-30).all()          # two roundings to bf16
 
 
+# whole heads in halves, of every width that has a kernel of its own, and a part of a head; heads that fill no warp, a part of a
+# second one, and several
 @pytest.mark.gpu
-def test_rope_reads_queries_beside_their_gates():
+@pytest.mark.parametrize("d,rot", [(64, 64), (128, 128), (256, 256), (128, 32)])
+@pytest.mark.parametrize("nq,nkv", [(1, 1), (6, 2), (29, 3)])
+def test_rope_reads_queries_beside_their_gates(d, rot, nq, nkv):
     from xllm_b200 import ops
     from xllm_b200.ops import reference
-    g = torch.Generator().manual_seed(0)
-    T, nq, nkv, d, rot = 7, 6, 2, 128, 32
+    g = torch.Generator().manual_seed(d + rot + nq)
+    T, page, pages = 23, 16, 4
     qkv = torch.randn(T, nq * 2 * d + 2 * nkv * d, generator=g).bfloat16().cuda()
-    w = [(0.1 * torch.randn(d, generator=g)).bfloat16().cuda() for _ in range(2)]
-    cs = reference.build_cos_sin_cache(rot, 64, 1e4, None, "cuda")
-    pos = torch.arange(T).cuda()
-    packed = torch.cat([qkv[:, :nq * 2 * d].view(T, nq, 2 * d)[..., :d].reshape(T, nq * d), qkv[:, nq * 2 * d:]], dim=1)
     # weights w + 1 that bf16 holds exactly: both ways add in fp32
-    w = [((1 + x) - 1) for x in w]
-    kw = dict(eps=1e-6, return_kv=True)
-    want = ops.rope_kv_write(packed, nq, nkv, d, pos, cs, rot, q_norm_w=w[0] + 1, k_norm_w=w[1] + 1, **kw)
-    got = ops.rope_kv_write(qkv, nq, nkv, d, pos, cs, rot, q_norm_w=w[0], k_norm_w=w[1], q_head_stride=2 * d, norm_offset=1.0, **kw)
-    for a, b in zip(got, want):
+    w = [((1 + (0.1 * torch.randn(d, generator=g)).bfloat16().cuda()) - 1) for _ in range(2)]
+    cs = reference.build_cos_sin_cache(rot, 64, 1e4, None, "cuda")
+    pos = torch.randint(0, 64, (T,), generator=g).cuda()
+    slots = torch.randperm(pages * page, generator=g)[:T].int().cuda()
+    slots[[3, T - 1]] = -1
+    packed = torch.cat([qkv[:, :nq * 2 * d].view(T, nq, 2 * d)[..., :d].reshape(T, nq * d), qkv[:, nq * 2 * d:]], dim=1)
+    outs = []
+    for rows, extra in ((packed, dict(q_norm_w=w[0] + 1, k_norm_w=w[1] + 1)),
+                        (qkv, dict(q_norm_w=w[0], k_norm_w=w[1], q_head_stride=2 * d, norm_offset=1.0))):
+        caches = [torch.full((pages, nkv, page, d), 7.0, device="cuda").bfloat16() for _ in range(2)]
+        outs.append([*ops.rope_kv_write(rows, nq, nkv, d, pos, cs, rot, slots=slots, k_cache=caches[0], v_cache=caches[1], eps=1e-6,
+                                        return_kv=True, **extra), *caches])
+    for a, b in zip(*outs):
         assert torch.equal(a, b)
+    q, k, v, k_cache, v_cache = outs[1]
+    for got, want in zip((q, k, v), reference.rope_kv(packed.double(), nq, nkv, d, pos, cs.double(), rot, (w[0] + 1).double(),
+                                                      (w[1] + 1).double(), 1e-6, False)):
+        # the normed value, and the result of two products, are rounded to bf16: 2^-9 at most each
+        assert (got.double() - want).norm() <= 2 ** -8 * want.norm()
+    for cache, dense in ((k_cache, k), (v_cache, v)):
+        at = torch.full_like(cache, 7.0)
+        for t, s in enumerate(slots.tolist()):
+            if s >= 0:
+                at[s // page, :, s % page] = dense[t]
+        assert torch.equal(cache, at)

@@ -51,9 +51,9 @@ def test_fp8(M, N, K):
     _close(fp8.block_scaled_mm(a, a_s, w, w_s), want, 2 ** -8)
 
 
-# more rows: single CTAs and pairs; rows, columns and K blocks that fill no tile, and more tiles than pairs
+# more rows, in tiles of 128: rows, columns and K blocks that fill no tile, and more tiles than SMs
 @pytest.mark.parametrize("M,N,K", [(130, 2048, 256), (300, 7168, 640), (922, 7168, 2048), (1000, 8200, 384), (2100, 4352, 256)])
-def test_fp8_pairs(M, N, K):
+def test_fp8_of_many_rows(M, N, K):
     test_fp8(M, N, K)
 
 

@@ -32,20 +32,27 @@ def _oracle(q, kc, vc, bt, cu, lens, scale, causal, window, keep, softcap, sink)
     return out
 
 
-@pytest.mark.parametrize("page", [16, 64, 128])
-@pytest.mark.parametrize("options", [{}, {"window": 100}, {"window": 200, "keep": 5}, {"softcap": 3.0}, {"softcap": 50.0, "window": 300},
-                                     {"causal": False}, {"sink": True}])
-@pytest.mark.parametrize("lens,behind", [([700, 300, 129, 385], [0, 0, 0, 0]), ([256, 1, 257, 900], [130, 77, 0, 511])])
-def test_two_tiles(lens, behind, options, page):
+def _case(lens, behind, page, nq=32, nkv=8):
     g = torch.Generator(device="cuda").manual_seed(sum(lens) + page)
-    nq, nkv, T = 32, 8, sum(lens)
+    T = sum(lens)
     kv = [a + b for a, b in zip(lens, behind)]
     per = max(-(-n // page) for n in kv)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
     q, kc, vc = rnd(T, nq, 128) * 2, rnd(len(lens) * per + 1, nkv, page, 128), rnd(len(lens) * per + 1, nkv, page, 128)
     bt = (1 + torch.randperm(len(lens) * per, device="cuda", generator=g)).view(len(lens), per).int()
     cu = torch.tensor([0] + lens, device="cuda").cumsum(0).int()
-    kvl = torch.tensor(kv, dtype=torch.int32, device="cuda")
+    return g, q, kc, vc, bt, cu, torch.tensor(kv, dtype=torch.int32, device="cuda")
+
+
+# the last three: prompts whose mean length lies below, at and above what two tiles a block are taken from
+@pytest.mark.parametrize("page", [16, 64, 128])
+@pytest.mark.parametrize("options", [{}, {"window": 100}, {"window": 200, "keep": 5}, {"softcap": 3.0}, {"softcap": 50.0, "window": 300},
+                                     {"causal": False}, {"sink": True}])
+@pytest.mark.parametrize("lens,behind", [([700, 300, 129, 385], [0, 0, 0, 0]), ([256, 1, 257, 900], [130, 77, 0, 511]),
+                                         ([100] * 9 + [300], [0, 40] * 5), ([130] * 7 + [242], [0] * 8), ([130] * 7 + [250], [0] * 8)])
+def test_two_tiles(lens, behind, options, page):
+    g, q, kc, vc, bt, cu, kvl = _case(lens, behind, page)
+    nq = q.shape[1]
     o = {"causal": True, "window": 0, "keep": 0, "softcap": 0.0, "sink": None, **options}
     if o["sink"]:
         o["sink"] = torch.randn(nq, device="cuda", generator=g) * 2
@@ -55,3 +62,27 @@ def test_two_tiles(lens, behind, options, page):
     assert (got.double() - want).norm() <= 2 ** -8 * want.norm()
     worst = (got.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
     assert float(worst.max()) <= 2 ** -6
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("lens,behind", [([700, 300, 129, 385], [0, 0, 0, 0]), ([256, 1, 257, 900], [130, 77, 0, 511]),
+                                         ([100] * 9 + [300], [0, 40] * 5)])
+def test_log_sum_exps(lens, behind, causal):
+    from xllm_b200.ops import _lib, xattn  # noqa: F401 (declares the entry point)
+    from xllm_b200.ops._lib import check, ptr, stream
+    _, q, kc, vc, bt, cu, kvl = _case(lens, behind, 16)
+    T, nq, nkv, out = q.shape[0], q.shape[1], kc.shape[1], torch.empty_like(q)
+    lse = torch.full((T, nq), 7.0, device="cuda")
+    check(_lib.load().xllm_paged_prefill_attn_tc_lse(ptr(out), out.stride(0), ptr(q), q.stride(0), T, ptr(kc), ptr(vc), kc.shape[0],
+                                                     ptr(bt), bt.stride(0), ptr(cu), ptr(kvl), len(lens), max(lens), nq, nkv, 16,
+                                                     128 ** -0.5, int(causal), 0, ptr(lse), stream()), "lse")
+    for i, n in enumerate(kvl.tolist()):
+        b, e = int(cu[i]), int(cu[i + 1])
+        k = kc[bt[i, :-(-n // 16)].long()].transpose(1, 2).reshape(-1, nkv, 128)[:n].double().repeat_interleave(nq // nkv, 1)
+        s = torch.einsum("nhd,thd->hnt", q[b:e].double(), k) * 128 ** -0.5
+        if causal:
+            pos = torch.arange(n - (e - b), n, device="cuda")[:, None]
+            s = s.masked_fill(torch.arange(n, device="cuda")[None] > pos, float("-inf"))
+        want = torch.logsumexp(s, dim=2).T * 1.4426950408889634
+        # scores in fp32 and exponentials of 2^-22: sums of up to 1400 positive terms
+        assert float((lse[b:e].double() - want).abs().max()) <= 1e-4

@@ -47,6 +47,15 @@ def test_xattention_matches_reference(lens, W, n_tail):
     assert err < 2e-2, err
 
 
+# as many rows and heads as the prompt kernel takes two tiles a block for
+@pytest.mark.parametrize("lens,W,n_tail", [([300, 57], 600, 2), ([1100], 1030, 1)])
+def test_xattention_of_wide_beams(lens, W, n_tail):
+    got, want = _case(lens, W, n_tail, cap=max(n_tail, 1), nq=32, nkv=8)
+    assert torch.isfinite(got).all()
+    err = (got - want).abs().max().item()
+    assert err < 2e-2, err
+
+
 def test_rec_engine_on_device_matches_exhaustive_beam():
     from xllm_b200 import LLM
     from xllm_b200.engine.rec import ItemTrie, RecEngine, item_logprob_reference, recommend_reference

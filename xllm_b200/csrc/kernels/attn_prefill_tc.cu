@@ -921,8 +921,11 @@ static int prefill_tc(void* out, int64_t o_stride, const void* q, int64_t q_stri
   p.lse = (float*)lse; p.sink = (const float*)sink; p.keep = window > 0 ? keep : 0; p.rows_kv = kv_ld > 0; p.cap = make_soft_cap(scale, softcap);
   // Two query tiles a CTA where such CTAs fill most SMs (the batch's rows bound their number; a captured step's grid holds more
   // sequences than there are).  32 heads, one B200: 500 rows behind 1024 tokens, 64 CTAs, 33 us against 26 us with one tile;
-  // 1024 rows, 128 CTAs, 25 us against 31 us.
-  if (out != nullptr && max_q_len > kBM && (total_q + 2 * kBM - 1) / (2 * kBM) * nq >= 128) {
+  // 1024 rows, 128 CTAs, 25 us against 31 us.  Not where most prompts have one tile, which then has half the softmax warps and
+  // nothing to alternate with; their lengths are on the device, their mean is known here.  One tile a CTA and two, us: 40 prompts
+  // of 100 rows and one of 300 78 and 84, behind 1000 tokens 194 and 233; 40 of 128 and one of 300 (mean 132) 80 and 84; 12 of 150
+  // rows 44 and 36; 30 of 110 and four of 500 (mean 156) 92 and 85; 20 of 100 and one of 2000 (mean 190) 148 and 130.
+  if (out != nullptr && max_q_len > kBM && (total_q + 2 * kBM - 1) / (2 * kBM) * nq >= 128 && total_q >= 144 * (int64_t)batch) {
     const dim3 grid((max_q_len + 2 * kBM - 1) / (2 * kBM), nq, batch);
     const auto kernel = softcap > 0.f ? prefill_tc_two_kernel<true> : prefill_tc_two_kernel<false>;
     kernel<<<grid, 384, Q2_SMEM, (cudaStream_t)stream>>>(tq, tk, tv, p);
