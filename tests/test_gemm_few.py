@@ -190,7 +190,8 @@ def test_activation_and_its_quantisation(rows, d, act):
 
 
 # (tokens, experts, chosen): one row tile after another up to pairs of CTAs, experts with more rows than a tile and with none
-@pytest.mark.parametrize("T,E,K", [(1, 8, 2), (9, 32, 4), (40, 16, 4), (64, 8, 2), (130, 8, 2), (447, 8, 2), (448, 8, 2), (1500, 8, 2)])
+@pytest.mark.parametrize("T,E,K", [(1, 8, 2), (9, 32, 4), (40, 16, 4), (64, 8, 2), (130, 8, 2), (447, 8, 2), (448, 8, 2), (1500, 8, 2),
+                                   (72, 16, 4), (73, 16, 4), (112, 16, 4), (113, 16, 4), (225, 16, 4), (527, 8, 2), (528, 8, 2)])
 @pytest.mark.parametrize("fp8_weights", [False, True])
 def test_expert_layer(T, E, K, fp8_weights):
     g = torch.Generator(device=DEV).manual_seed(T * E)

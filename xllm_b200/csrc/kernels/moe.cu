@@ -3,7 +3,7 @@
 //   moe_route    : softmax / sigmoid scoring (+ selection bias), group-limited top-k
 //                  (n_group / topk_group), renormalisation, routed scaling; emits expert ids,
 //                  weights, per-expert counts and each token's slot inside its expert
-//   moe_offsets  : padded exclusive scan of the counts (segments start on 128-row tiles, so a
+//   moe_offsets  : padded exclusive scan of the counts (segments start on row tiles, so a
 //                  GEMM tile never straddles two experts) + the tile -> expert table the grouped
 //                  GEMM walks
 //   moe_permute  : gather token rows into expert-major order
@@ -329,10 +329,6 @@ XLLM_API int xllm_moe_offsets_tile(void* counts, void* offsets, void* tile_exper
   launch_pdl(moe_offsets_kernel, dim3(1), dim3(256), 0, (cudaStream_t)stream, (int32_t*)counts, (int32_t*)offsets,
              (int32_t*)tile_expert, (int32_t*)meta, E, max_tiles, expert_begin, tile);
   return XLLM_LAUNCH_CHECK();
-}
-XLLM_API int xllm_moe_offsets(void* counts, void* offsets, void* tile_expert, void* meta, int E, int max_tiles,
-                              int expert_begin, void* stream) {
-  return xllm_moe_offsets_tile(counts, offsets, tile_expert, meta, E, max_tiles, expert_begin, xllm::kMoeTile, stream);
 }
 
 static int moe_permute(void* xp, void* rows, const void* x, const void* topk_ids, const void* slot, const void* offsets, int T,

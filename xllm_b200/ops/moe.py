@@ -17,7 +17,6 @@ from .fp8 import FEW_K
 
 _lib.register_signature("xllm_moe_route", [P, I, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P])
 _lib.register_signature("xllm_moe_route_ld", [P, L, I, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P])
-_lib.register_signature("xllm_moe_offsets", [P, P, P, P, I, I, I, P])
 _lib.register_signature("xllm_moe_offsets_tile", [P, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_moe_permute_fp8", [P, P, P, P, P, P, P, P, I, I, I, I, P])
 _lib.register_signature("xllm_gemm_bf16_grouped_few", [P, P, P, P, I, I, I, I, I, L, L, I, F, F, P])
@@ -70,21 +69,27 @@ def fused_moe_reference(x, logits, w_gate_up, w_down, top_k, scoring="softmax", 
 
 
 MIN_TILE = 16
-MANY_ROWS = 112          # per expert: from here on, tiles of 256 rows
+FEW_ROWS = ((16, 18), (32, 28), (64, 56))      # a tile's rows, and up to how many rows per expert on average it is taken
+MANY_ROWS = 132                                # from here on, tiles of 256 rows
 
 
 def row_tile(T, top_k, n_experts):
     """Rows of a tile of the grouped products, none of which two experts share.  With few rows per expert the products are
     bound by the experts' weights, and small tiles (csrc/kernels/gemm_few.cu) leave out the rows that are not there; an
-    expert with more rows than a tile reads its weights again for the next, from L2.  So: the smallest tile that holds
-    about 2.5 times the average, 128 (gemm_tcgen05.cu) beyond.  Many rows are bound by the operands' way from L2: a CTA
-    pair's tile of 256 reads 256 rows of operands per SM and K block for what takes single CTAs' 128-row tiles 384, so it
-    is the better one for experts of more than 128 rows, up to 256 of which it pads to as much as two of the others.
-    Measured (one B200, 128 experts of 768, a layer's two products): 16 tokens 189 us in tiles of 128, 126 us in tiles of
-    16; 3066 tokens (192 rows per expert) 306 us in tiles of 128, 285 us in pairs' tiles of 256."""
+    expert with more rows than a tile reads its weights again for the next, from L2, so a tile lasts while most experts fill
+    one.  Tiles of 128 are those of gemm_tcgen05.cu.  Many rows are bound by the operands' way from L2: a CTA pair's tile of
+    256 reads 256 rows of operands per SM and K block for what takes single CTAs' 128-row tiles 384, so it is the better one
+    for experts of more than 128 rows.
+
+    Measured (one B200, us a layer; A: 128 experts of 768 x 2048, B: 32 of 2048 x 7168 in e4m3, C: 8 of 14336 x 4096), by rows
+    per expert, in the two tiles between which the line lies:
+      16 and 32   at 16: A 240, 250  B 297, 303  C 471, 484   at 20: A 254, 252  B 313, 303  C 532, 485
+      32 and 64   at 24: A 254, 268  B 305, 340  C 483, 487   at 32: A 287, 268  B 334, 358  C 539, 489
+      64 and 128  at 48: A 274, 276  B 367, 453               at 64: A 326, 279  B 422, 457  C 520, 518
+      128 and 256 at 128: A 322, 332  C 633, 581              at 136: A 351, 334  C 655, 580"""
     if T * top_k >= MANY_ROWS * n_experts:
         return 256
-    return next((t for t in (16, 32, 64) if T * top_k * 5 <= 2 * t * n_experts), 128)
+    return next((t for t, most in FEW_ROWS if T * top_k <= most * n_experts), 128)
 
 
 class MoeWorkspace:
