@@ -21,10 +21,13 @@
 // Every mbarrier wait is bounded (clock64 budget); on expiry the kernel raises an error word in
 // global memory, all roles leave their loops, TMEM is released and the kernel returns normally.
 #include "common.cuh"
+#include "tc_common.cuh"
 #include <cuda.h>
 #include <cstdlib>
 
 namespace xllm {
+
+using tc::elect_one;
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;  // 64 bf16 = 128 bytes = one swizzle row
@@ -153,16 +156,6 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
                : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-// One lane of a converged warp.  The producer and MMA warps run their loops with all 32 lanes and
-// only predicate the TMA / tcgen05 instructions on the elected lane: loop state, shared-memory
-// addresses and descriptors then stay warp-uniform, which is what these instructions take as
-// operands (a loop run by a single lane under divergence pays a register-file round trip per
-// operand: measured ~120 cycles per tcgen05.mma issue against ~30 here).
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-  return pred != 0;
-}
 // Whole-warp bounded wait: every lane polls, the verdict is made uniform.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));

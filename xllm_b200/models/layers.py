@@ -595,7 +595,9 @@ class DenseMLP(Module):
         if gu.interleaved:
             from ..ops import gemm, gemm_tcgen05
             # (in between, narrower tiles and a kernel of its own for the activation are quicker)
-            if (x.is_cuda and x.dim() == 2 and (x.shape[0] > 512 or gemm_tcgen05.few_rows(x.shape[0], gu.weight.shape[0])) and gemm.gemm_mode() != "cublas" and gu.weight.shape[0] % 256 == 0
+            rows, width = x.shape[0], gu.weight.shape[0]
+            fused = rows > 512 or gemm_tcgen05.few_rows(rows, width)
+            if (fused and x.is_cuda and x.dim() == 2 and width % 256 == 0 and gemm.gemm_mode() != "cublas"
                     and gemm_tcgen05.supported(x, gu.weight)):
                 return gemm_tcgen05.gemm_act_mul(x, gu.weight, self.act)
             y = gu(x)
