@@ -288,9 +288,9 @@ __global__ void __launch_bounds__(256, 2) gdn_step_kernel(GdnParams p) {
 //
 // Every decay is at most 1.  y and v are bf16 as the convolution leaves them, so that their products on the tensor cores are
 // exact and accumulate in fp32; S, U, M and P are fp32 values as three bf16 terms (24 bits), of which products below 2^-24 of
-// the largest are left out.  (A chunk with anything that is not finite goes token by token.)  gdn_prep_kernel makes M, P and the factors, all chunks side by side; gdn_chunk_kernel walks the
-// chunks of a sequence: a warp owns 16 state columns for all of dk as accumulators of S^T, which are the A operand of S^T Y^T
-// without leaving the registers, as U^T is of the products behind it.
+// the largest are left out.  (A chunk with anything that is not finite goes token by token.)  gdn_prep_kernel makes M, P and the
+// factors, all chunks side by side; gdn_chunk_kernel walks the chunks of a sequence: a warp owns 16 state columns for all of dk as
+// accumulators of S^T, which are the A operand of S^T Y^T without leaving the registers, as U^T is of the products behind it.
 //
 // Token by token in fp32 (states in registers, no barriers) the walk took 600 us for four prompts of 1024, 549, 842 and 366
 // tokens, 32 heads of 128 x 128 (one B200), some 1100 cycles a token in a chain of product, exchange, product; in chunks it

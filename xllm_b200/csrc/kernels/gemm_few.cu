@@ -21,9 +21,9 @@
 //         clusters: a step of two latent layers 0.02 to 0.03 from the same rows' among many).
 //
 // Measured (one B200, 16 rows, before: gemm_fp8_block_kernel): 7168 x 16384 fp8 (117 MB of weights, 18 us at the copy rate)
-// 56 -> 29 us, 1536 x 7168 25 -> 10 us, 7168 x 18432 63 -> 32 us; 32 experts, eight of
-// which each row chose, 4096 x 7168 214 -> 163 us (143 at the copy rate) and 7168 x 2048 186 -> 92 us (72).  bf16, one row (before: split-K in gemm_tcgen05.cu, and the activation's own kernel): 4096 x 4096 13 -> 9 us,
-// gated 24576 x 4096 44 -> 39 us (31 at the copy rate), 4096 x 12288 26 -> 20 us.
+// 56 -> 29 us, 1536 x 7168 25 -> 10 us, 7168 x 18432 63 -> 32 us; 32 experts, of which every row chose eight, 4096 x 7168 214 -> 163
+// us (143 at the copy rate) and 7168 x 2048 186 -> 92 us (72).  bf16, one row (before: split-K in gemm_tcgen05.cu, and the
+// activation's own kernel): 4096 x 4096 13 -> 9 us, gated 24576 x 4096 44 -> 39 us (31 at the copy rate), 4096 x 12288 26 -> 20 us.
 //
 // Every mbarrier wait is bounded; on expiry all roles leave, tensor memory is released and an error word is set
 // (xllm_gemm_few_error_status).
